@@ -186,14 +186,12 @@ __device__ __forceinline__ void pair_flux_mhd(const KParams& P, double ch, const
       for (int d = 0; d < 3; ++d) F[5 + d] = F[5 + d] + phiHat * m[d];
       F[8] = 0.5 * ch * (qbL + qbR);
     } else if constexpr (VF == 10) {  // EntropyAndKinEnergyConservingFluxVec_Derigs :761-848
-      double nr, dr, nb, db;
-      ln_mean_nd(L, R, 0, 12, nr, dr);
-      ln_mean_nd(L, R, 1, 13, nb, db);
       const double sr = L[0] + R[0], sb = L[1] + R[1];
-      const double inv = 1. / (dr * nb * sb);
-      const double rhoLN = nr * nb * sb * inv;    // LN(rho)
-      const double sbLN = db * dr * sb * inv;     // 1/LN(beta)
-      const double rsb = sr * dr * nb * inv;      // (rho_L+rho_R)/(beta_L+beta_R)
+      const double inv = rcp_nr(sr * sb);
+      const double isr = sb * inv, isb = sr * inv;          // 1/sr, 1/sb
+      const double rhoLN = ln_mean(L, R, 0, 12, sr, isr);   // LN(rho)
+      const double sbLN = inv_ln_mean(L, R, 1, 13, isb);    // 1/LN(beta)
+      const double rsb = sr * isb;                          // (rho_L+rho_R)/(beta_L+beta_R)
       double vA[3], BA[3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) { vA[d] = 0.5 * (L[2 + d] + R[2 + d]); BA[d] = 0.5 * (L[5 + d] + R[5 + d]); }
@@ -215,12 +213,10 @@ __device__ __forceinline__ void pair_flux_mhd(const KParams& P, double ch, const
       F[4] = F[0] * 0.5 * (P.sKappaM1 * sbLN - 0.5 * (L[9] + R[9])) + (vA[0] * F[1] + vA[1] * F[2] + vA[2] * F[3]) +
              smu0 * (sB - 0.25 * b2v + 0.5 * (L[11] + R[11]) * Bm + F[8] * psiA - (ch * 0.5) * pB);
     } else if constexpr (VF == 12) {  // EntropyAndKinEnergyConservingFluxVec_FloGor :970-1074
-      double nr, dr, ne, de;
-      ln_mean_nd(L, R, 0, 10, nr, dr);
-      ln_mean_nd(L, R, 2, 11, ne, de);
-      const double inv = 1. / (dr * ne);
-      const double rhoLN = nr * ne * inv;
-      const double ieT = L[2] * R[2] * de * dr * inv;  // e_L e_R / LN(e)
+      const double sr = L[0] + R[0], se = L[2] + R[2];
+      const double inv = rcp_nr(sr * se);
+      const double rhoLN = ln_mean(L, R, 0, 10, sr, se * inv);
+      const double ieT = L[2] * R[2] * inv_ln_mean(L, R, 2, 11, sr * inv);  // e_L e_R / LN(e)
       double vA[3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) vA[d] = 0.5 * (L[3 + d] + R[3 + d]);

@@ -6,22 +6,20 @@
 // VolumeFluxAverageVec family (src/equation/navierstokes/flux_average.f90); results agree with
 // the reference formulas to roundoff:
 //  - the logarithmic mean LN_MEAN (flux_average.f90:1945-1965) keeps its series branch for
-//    f^2 = ((b-a)/(b+a))^2 < 1e-4, written as 0.5 s^7 / (s^6 + s^4 d^2/3 + s^2 d^4/5 + d^6/7)
-//    (s = a+b, d = b-a; identical to (a+b)*52.5/(105+35u+21u^2+15u^3)), and otherwise uses
-//    (b-a)/(log b - log a) with per-node logarithms;
-//  - every log mean is kept as a (numerator, denominator) pair and all divisions of one pair
-//    flux are merged into a single reciprocal (rcp_nr).
+//    u = ((b-a)/(b+a))^2 < 1e-4, as a product with a series in u (ln_mean, inv_ln_mean), and
+//    otherwise uses (b-a)/(log b - log a) with per-node logarithms;
+//  - the divisions of one pair flux are merged into a single reciprocal (rcp_nr).
 #pragma once
 #include "common.cuh"
 
 namespace fluxo {
 
-// Reciprocal of x > 0 (normal, not huge) for the pair fluxes: the hardware's approximate reciprocal
+// Reciprocal of x (nonzero, normal, not huge) for the pair fluxes: the hardware's approximate reciprocal
 // (PTX rcp.approx.ftz.f64) refined by two Newton-Raphson steps for f(y) = 1/y - x,
 // y <- y + y (1 - x y), each computed with fused multiply-adds.  The approximation's relative error
 // is squared by every step, so two steps reach double precision (within an ulp of the rounded
-// quotient); the denominators here are products of densities, inverse temperatures and their log
-// means, far from zero and from overflow.  It replaces the longer IEEE division sequence (one per pair).
+// quotient); the denominators here are products of the sums of densities and inverse temperatures
+// (off the log mean's series branch: their differences), far from zero and from overflow.  It replaces the longer IEEE division sequence (one per pair).
 __device__ __forceinline__ double rcp_nr(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -31,31 +29,22 @@ __device__ __forceinline__ double rcp_nr(double x) {
   return fma(y, e, y);
 }
 
-// log mean of (a, b) as num/den given la = log(a), lb = log(b)
-__device__ __forceinline__ void ln_mean_nd(double a, double b, double la, double lb, double& num, double& den) {
-  const double d = b - a, s = b + a;
-  const double d2 = d * d, s2 = s * s;
-  const double qs = s2 * (s2 * (s2 + d2 * (1. / 3.)) + d2 * d2 * (1. / 5.)) + d2 * d2 * d2 * (1. / 7.);
-  const bool series = d2 < 1.0e-4 * s2;
-  num = series ? 0.5 * s * (s2 * s2 * s2) : d;
-  den = series ? qs : (lb - la);
+// Logarithmic mean (LN_MEAN) of a = L[i] and b = R[i] and its reciprocal, given s = a + b and is = 1/s.
+// With u = ((b-a)/s)^2 < 1e-4 the mean is s/2 / (1 + u/3 + u^2/5 + u^3/7); ln_mean multiplies by the
+// series of that reciprocal, 1 - u/3 - 4u^2/45 - 44u^3/945 (the next term is below 1e-17), and
+// inv_ln_mean by the polynomial itself, so neither divides: one reciprocal 1/(s_a s_b) serves both means
+// of a pair.  Off the series branch the mean is (b-a)/(log b - log a); the logarithms log a = L[il],
+// log b = R[il] are read only there (R usually points into shared memory: in smooth flows nearly every
+// pair takes the series branch).
+__device__ __forceinline__ double ln_mean(const double* L, const double* R, int i, int il, double s, double is) {
+  const double d = R[i] - L[i], f = d * is, u = f * f;
+  if (u < 1.0e-4) return s * fma(u, fma(u, fma(u, -22. / 945., -2. / 45.), -1. / 6.), 0.5);
+  return d * rcp_nr(R[il] - L[il]);
 }
-
-// log mean of (a, b) = (L[i], R[i]) as num/den; the logarithms log a = L[il], log b = R[il] are read
-// only off the series branch (R usually points into shared memory: in smooth flows nearly every
-// pair takes the series branch, so its two logarithm loads are skipped)
-__device__ __forceinline__ void ln_mean_nd(const double* L, const double* R, int i, int il, double& num,
-                                           double& den) {
-  const double a = L[i], b = R[i];
-  const double d = b - a, s = b + a;
-  const double d2 = d * d, s2 = s * s;
-  if (d2 < 1.0e-4 * s2) {
-    num = 0.5 * s * (s2 * s2 * s2);
-    den = s2 * (s2 * (s2 + d2 * (1. / 3.)) + d2 * d2 * (1. / 5.)) + d2 * d2 * d2 * (1. / 7.);
-  } else {
-    num = d;
-    den = R[il] - L[il];
-  }
+__device__ __forceinline__ double inv_ln_mean(const double* L, const double* R, int i, int il, double is) {
+  const double d = R[i] - L[i], f = d * is, u = f * f;
+  if (u < 1.0e-4) return is * fma(u, fma(u, fma(u, 2. / 7., 2. / 5.), 2. / 3.), 2.);
+  return (R[il] - L[il]) * rcp_nr(d);
 }
 
 // Record of a node in shared memory: NQ flux quantities at [0, NQ), the metric terms Ja^1..Ja^3
@@ -213,8 +202,7 @@ __device__ __forceinline__ void pair_flux(const KParams& P, const double* L, con
       F[3] = F[0] * wH + m3 * p1;
       F[4] = F[0] * 0.5 * (P.sKappaM1 * sbM - (L[5] + R[5])) + uH * F[1] + vH * F[2] + wH * F[3];
     } else if constexpr (VF == 7) {  // ggFluxVec :1575-1653 (halves)
-      double nb, db;
-      ln_mean_nd(L, R, 5, 7, nb, db);
+      const double sbHat = inv_ln_mean(L, R, 5, 7, rcp_nr(L[5] + R[5]));
       const double rhoM = L[0] + R[0];
       const double uH = L[1] + R[1], vH = L[2] + R[2], wH = L[3] + R[3];
       const double p1 = L[4] + R[4];
@@ -223,7 +211,7 @@ __device__ __forceinline__ void pair_flux(const KParams& P, const double* L, con
       F[1] = F[0] * uH + m1 * p1;
       F[2] = F[0] * vH + m2 * p1;
       F[3] = F[0] * wH + m3 * p1;
-      F[4] = F[0] * 0.5 * (P.sKappaM1 * (db * rcp_nr(nb)) - (L[6] + R[6])) + uH * F[1] + vH * F[2] + wH * F[3];
+      F[4] = F[0] * 0.5 * (P.sKappaM1 * sbHat - (L[6] + R[6])) + uH * F[1] + vH * F[2] + wH * F[3];
     } else if constexpr (VF == 8) {  // KennedyAndGruberFluxVec2 :857-929 (halves)
       const double uH = L[1] + R[1], vH = L[2] + R[2], wH = L[3] + R[3];
       const double p1 = L[4] + R[4];
@@ -245,14 +233,12 @@ __device__ __forceinline__ void pair_flux(const KParams& P, const double* L, con
       F[3] = q * wH + m3 * p1;
       F[4] = q * HH;
     } else if constexpr (VF == 5) {  // EntropyAndEnergyConservingFluxVec :1277-1356
-      double nr, dr, nb, db;
-      ln_mean_nd(L, R, 0, 6, nr, dr);
-      ln_mean_nd(L, R, 4, 7, nb, db);
       const double sr = L[0] + R[0], sb = L[4] + R[4];
-      const double inv = rcp_nr(dr * sb * nb);
-      const double rhoHat = nr * sb * nb * inv;      // LN(rho)
-      const double p1 = 0.5 * sr * dr * nb * inv;    // 0.5*rho_mean/beta_mean
-      const double sbHat = db * dr * sb * inv;       // 1/LN(beta)
+      const double inv = rcp_nr(sr * sb);
+      const double isr = sb * inv, isb = sr * inv;            // 1/sr, 1/sb
+      const double rhoHat = ln_mean(L, R, 0, 6, sr, isr);     // LN(rho)
+      const double sbHat = inv_ln_mean(L, R, 4, 7, isb);      // 1/LN(beta)
+      const double p1 = 0.5 * sr * isb;                       // 0.5*rho_mean/beta_mean
       const double uH = L[1] + R[1], vH = L[2] + R[2], wH = L[3] + R[3];  // records hold u/2, v/2, w/2
       const double q = uH * m1 + vH * m2 + wH * m3;
       F[0] = rhoHat * q;
@@ -261,19 +247,16 @@ __device__ __forceinline__ void pair_flux(const KParams& P, const double* L, con
       F[3] = F[0] * wH + m3 * p1;
       F[4] = F[0] * 0.5 * (P.sKappaM1 * sbHat - (L[5] + R[5])) + uH * F[1] + vH * F[2] + wH * F[3];
     } else if constexpr (VF == 10) {  // TwoPointEntropyConservingFluxVec :574-673
-      double n1, d1, n5, d5;
-      ln_mean_nd(L, R, 0, 5, n1, d1);
-      ln_mean_nd(L, R, 4, 6, n5, d5);
-      const double z1M = 0.5 * (L[0] + R[0]);
-      const double inv = rcp_nr(d5 * z1M * n1);
-      const double z5LN = n5 * z1M * n1 * inv;
-      const double sz1M = d5 * n1 * inv;
-      const double ratio = n5 * d1 * z1M * inv;  // z5LN / z1LN
-      const double rhoHat = z1M * z5LN;
-      const double uH = 0.5 * (L[0] * L[1] + R[0] * R[1]) * sz1M;
-      const double vH = 0.5 * (L[0] * L[2] + R[0] * R[2]) * sz1M;
-      const double wH = 0.5 * (L[0] * L[3] + R[0] * R[3]) * sz1M;
-      const double p1 = 0.5 * (L[4] + R[4]) * sz1M;
+      const double s1 = L[0] + R[0], s5 = L[4] + R[4];
+      const double inv = rcp_nr(s1 * s5);
+      const double is1 = s5 * inv, is5 = s1 * inv;               // 1/s1, 1/s5
+      const double z5LN = ln_mean(L, R, 4, 6, s5, is5);
+      const double ratio = z5LN * inv_ln_mean(L, R, 0, 5, is1);  // z5LN / z1LN
+      const double rhoHat = 0.5 * s1 * z5LN;
+      const double uH = (L[0] * L[1] + R[0] * R[1]) * is1;
+      const double vH = (L[0] * L[2] + R[0] * R[2]) * is1;
+      const double wH = (L[0] * L[3] + R[0] * R[3]) * is1;
+      const double p1 = s5 * is1;
       const double q = uH * m1 + vH * m2 + wH * m3;
       F[0] = rhoHat * q;
       F[1] = F[0] * uH + m1 * p1;
@@ -281,12 +264,10 @@ __device__ __forceinline__ void pair_flux(const KParams& P, const double* L, con
       F[3] = F[0] * wH + m3 * p1;
       F[4] = 0.5 * (q * P.kappaP1 * P.sKappaM1 * ratio + uH * F[1] + vH * F[2] + wH * F[3]);
     } else if constexpr (VF == 32) {  // RanochaFluxVec :1876-1929
-      double nr, dr, ns, ds;
-      ln_mean_nd(L, R, 0, 6, nr, dr);
-      ln_mean_nd(L, R, 5, 7, ns, ds);
-      const double inv = rcp_nr(dr * ns);
-      const double rhoLN = nr * ns * inv;
-      const double srspM = ds * dr * inv;  // 1/LN(rho/p)
+      const double sr = L[0] + R[0], ss = L[5] + R[5];
+      const double inv = rcp_nr(sr * ss);
+      const double rhoLN = ln_mean(L, R, 0, 6, sr, ss * inv);
+      const double srspM = inv_ln_mean(L, R, 5, 7, sr * inv);  // 1/LN(rho/p)
       const double va1 = 0.5 * (L[1] + R[1]), va2 = 0.5 * (L[2] + R[2]), va3 = 0.5 * (L[3] + R[3]);
       const double v2zip = 0.5 * (L[1] * R[1] + L[2] * R[2] + L[3] * R[3]);
       const double pavg = 0.5 * (L[4] + R[4]);
