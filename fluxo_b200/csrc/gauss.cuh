@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(NP * NP * NP, NP == 8 ? 2 : 1) surf_kernel(KPa
     double FB[5], mN[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) mN[c] = dir == 0 ? m[c] : (dir == 1 ? m[3 + c] : m[6 + c]);  // registers
-    pair_flux<VF>(P, rN, o, mN, o + NQ, FB);
+    pair_flux<VF>(P, rN, o, rN, o, mN, o + NQ, FB);
 #pragma unroll
     for (int v = 0; v < 5; ++v) sB[v * NP3 + t] = FB[v] * sLm[l];
     __syncthreads();

@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(NP * NP * NP, surf_mhd_minb<NP>()) surf_mhd_ke
 #pragma unroll
     for (int c = 0; c < 3; ++c) mN[c] = dir == 0 ? m[c] : (dir == 1 ? m[3 + c] : m[6 + c]);
     double FB[NV9], FC[NV9];
-    mhd::pair_flux_mhd<VF>(P, ch, rN, o, mN, o + NQ, FB);
+    mhd::pair_flux_mhd<VF>(P, ch, rN, o, rN, o, mN, o + NQ, FB);
 #pragma unroll
     for (int v = 0; v < NV9; ++v) FC[v] = FB[v];
     if (NC != 0) {

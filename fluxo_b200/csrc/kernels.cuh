@@ -201,12 +201,90 @@ __host__ __device__ constexpr size_t vol_smem_bytes() {
   return sizeof(double) * (size_t)(2 * NP * NP + EPB * (VolRec<VF>::RS + 5) * vol_pad_slots<NP, LPW>());
 }
 
+// Node epilogue of the volume kernels: from the split-form volume integral ut of node t of element e
+// (state u, ElemToSide e2s in shared memory) to Ut (stage 0) or the LSERK update: NFVSE blending, viscous
+// volume integral, surface integral, Jacobian, source.
+template <int NP, bool VISC>
+__device__ __forceinline__ void vol_finish_node(const KParams& P, int e, int t, const double* u, double* ut,
+                                                const int* e2s) {
+  constexpr int NP3 = NP * NP * NP, N = NP - 1, NPT = NP * NP;
+  if (P.nfvse) {  // VolInt_NFVSE (nfvse.f90:475-565): blend with alpha * F_FV of the subcell FV kernel
+    const double a = P.alpha[e];
+    const double* FV = P.fv + (size_t)e * 5 * NP3 + t;
+    if (P.nfvseCorr) {  // F_FV of every element; FFV_m_FDG = (F_FV - Ut) (-sJ) for the correction
+      const double sjn = P.sJ[(size_t)e * NP3 + t];
+      double* FF = P.ffvmfdg + 5 * ((size_t)e * NP3 + t);
+#pragma unroll
+      for (int v = 0; v < 5; ++v) {
+        const double f = FV[v * NP3];
+        FF[v] = (f - ut[v]) * (-sjn);
+        ut[v] = (1. - a) * ut[v] + a * f;
+      }
+    } else if (a > 4.440892098500626e-16) {
+#pragma unroll
+      for (int v = 0; v < 5; ++v) ut[v] = (1. - a) * ut[v] + FV[v * NP3];
+    }
+  }
+  if constexpr (VISC) {  // viscous volume integral (volint.f90:228-271), computed by the lifting kernel
+    const double* V = P.utvisc + (size_t)e * 4 * NP3 + t;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) ut[1 + v] += V[v * NP3];
+  }
+  if (P.utsurf) {  // Gauss nodes: the surface integral of every node, formed by the surface kernel
+    const double* S = P.utsurf + (size_t)e * 5 * NP3 + t;
+#pragma unroll
+    for (int v = 0; v < 5; ++v) ut[v] += S[v * NP3];
+  } else {  // surface integral at the boundary nodes (LGL)
+    const int i = t % NP, j = (t / NP) % NP, k = t / NPT;
+    int sides[3];
+    const int ns = boundary_sides(i, j, k, N, sides);
+    const double lh = P.basis->LhatM0;
+    for (int z = 0; z < ns; ++z) {
+      const int s = sides[z], side = e2s[2 * (s - 1)], flip = e2s[2 * (s - 1) + 1];
+      const int pt = node_side_point(N, s, flip, i, j, k);
+      const double* F = P.flux + (size_t)side * 5 * NPT + pt;
+      const double sg = (flip == 0) ? lh : -lh;
+#pragma unroll
+      for (int v = 0; v < 5; ++v) ut[v] += sg * F[v * NPT];
+    }
+  }
+  // Ut = -Ut*sJ  (+ source)
+  const double sj = P.sJ[(size_t)e * NP3 + t];
+  const double tStage = P.dtDev ? (P.dtDev[1] + P.rkC * P.dtDev[0]) : P.t;
+#pragma unroll
+  for (int v = 0; v < 5; ++v) ut[v] = ut[v] * (-sj);
+  if (P.source) {  // CalcSource CASE(4), equation.f90:1000-1024
+    const double* x = P.xGP + 3 * ((size_t)e * NP3 + t);
+    double arg = P.srcOmega * (x[0] + x[1] + x[2] - tStage);
+    double c = cos(arg), sn = sin(arg), s2 = 2. * sn * c;
+    ut[0] += P.srcTmp[0] * c;
+    double mm = P.srcTmp[1] * c + P.srcTmp[2] * s2;
+    ut[1] += mm; ut[2] += mm; ut[3] += mm;
+    ut[4] += P.srcTmp[3] * c + P.srcTmp[4] * s2 + P.srcTmp[5] * sn;
+  }
+  const size_t o = 5 * ((size_t)e * NP3 + t);
+  if (P.stage == 0) {
+#pragma unroll
+    for (int v = 0; v < 5; ++v) P.Ut[o + v] = ut[v];
+  } else {
+    // LSERK-2reg stage: Ut_tmp = Ut - A*Ut_tmp (stage 1: Ut_tmp = Ut); U = U + b*dt*Ut_tmp
+    const double dt = stage_dt(P, e);
+    const double bdt = P.rkB * dt;
+#pragma unroll
+    for (int v = 0; v < 5; ++v) {
+      double tmp = (P.stage == 1) ? ut[v] : ut[v] - P.UtTmp[o + v] * P.rkA;
+      P.UtTmp[o + v] = tmp;
+      P.U[o + v] = u[v] + tmp * bdt;
+    }
+  }
+}
+
 template <int NP, int VF, bool VISC, int EPB, int LPW, int MINB, int OWNSM>
 __global__ void __launch_bounds__(VolShape<NP, EPB, LPW>::THREADS, VolShape<NP, EPB, LPW, MINB>::MINB)
 volume_kernel(KParams P) {
   if (halted(P)) return;
-  constexpr int NP3 = NP * NP * NP, N = NP - 1, NPT = NP * NP;
-  constexpr int RS = VolRec<VF>::RS, NQ = VolRec<VF>::NQ;
+  constexpr int NP3 = NP * NP * NP, NPT = NP * NP;
+  constexpr int RS = VolRec<VF>::RS, NF = VolRec<VF>::NF;
   static_assert(LPW > 0 ? (32 / LPW >= NP) : (32 % NP == 0), "a line must fit its lanes of one warp");
   extern __shared__ double smem[];
   double* sDvs = smem;         // Dvolsurf(i,l) at [i*NP+l]
@@ -285,8 +363,8 @@ volume_kernel(KParams P) {
       const int base = dir == 0 ? NP * (la + NP * lb) : (dir == 1 ? la + NPT * lb : la + NP * lb);
       const int own = base + p * stride, os = vol_pad<NP, LPW>(own);
       // own record: held in registers for all rounds, or (OWNSM) read from shared memory in every
-      // round, which frees 2*(NQ+3) registers
-      double ro[NQ], mo[3], racc[5] = {0., 0., 0., 0., 0.};
+      // round, which frees 2*(NF+3) registers
+      double ro[NF], mo[3], racc[5] = {0., 0., 0., 0., 0.};
       if (!OWNSM && lv) {
         load_rec<VF>(prec + os * RS, ro);
         load_metric<VF>(prec + os * RS, dir, mo);
@@ -302,7 +380,7 @@ volume_kernel(KParams P) {
         if (active) {
           // the partner's record is read in place (the log-mean logarithms only when needed)
           const double* rq = prec + vol_pad<NP, LPW>(base + q * stride) * RS;
-          pair_flux<VF>(P, rOwn, rq, mOwn, rq + VolRec<VF>::MO + 3 * dir, F);
+          pair_flux<VF>(P, rOwn, rq, prec + os * RS, rq, mOwn, rq + VolRec<VF>::MO + 3 * dir, F);
         }
         const double dOwn = sDvs[p * NP + q], dPart = sDvs[q * NP + p];
         int src = p - d;
@@ -323,78 +401,257 @@ volume_kernel(KParams P) {
       __syncthreads();
     }
   }
+  if (!valid) return;
   double ut[5];
 #pragma unroll
-  for (int v = 0; v < 5; ++v) ut[v] = valid ? acc[vol_pad<NP, LPW>(t) * 5 + v] : 0.;
-  if (!valid) return;
-  if (P.nfvse) {  // VolInt_NFVSE (nfvse.f90:475-565): blend with alpha * F_FV of the subcell FV kernel
-    const double a = P.alpha[e];
-    const double* FV = P.fv + (size_t)e * 5 * NP3 + t;
-    if (P.nfvseCorr) {  // F_FV of every element; FFV_m_FDG = (F_FV - Ut) (-sJ) for the correction
-      const double sjn = P.sJ[(size_t)e * NP3 + t];
-      double* FF = P.ffvmfdg + 5 * ((size_t)e * NP3 + t);
-#pragma unroll
-      for (int v = 0; v < 5; ++v) {
-        const double f = FV[v * NP3];
-        FF[v] = (f - ut[v]) * (-sjn);
-        ut[v] = (1. - a) * ut[v] + a * f;
-      }
-    } else if (a > 4.440892098500626e-16) {
-#pragma unroll
-      for (int v = 0; v < 5; ++v) ut[v] = (1. - a) * ut[v] + FV[v * NP3];
-    }
-  }
-  if constexpr (VISC) {  // viscous volume integral (volint.f90:228-271), computed by the lifting kernel
-    const double* V = P.utvisc + (size_t)e * 4 * NP3 + t;
-#pragma unroll
-    for (int v = 0; v < 4; ++v) ut[1 + v] += V[v * NP3];
-  }
-  if (P.utsurf) {  // Gauss nodes: the surface integral of every node, formed by the surface kernel
-    const double* S = P.utsurf + (size_t)e * 5 * NP3 + t;
-#pragma unroll
-    for (int v = 0; v < 5; ++v) ut[v] += S[v * NP3];
-  } else {  // surface integral at the boundary nodes (LGL)
-    const int i = t % NP, j = (t / NP) % NP, k = t / NPT;
-    int sides[3];
-    const int ns = boundary_sides(i, j, k, N, sides);
-    const double lh = P.basis->LhatM0;
-    for (int z = 0; z < ns; ++z) {
-      const int s = sides[z], side = sE2S[eb][2 * (s - 1)], flip = sE2S[eb][2 * (s - 1) + 1];
-      const int pt = node_side_point(N, s, flip, i, j, k);
-      const double* F = P.flux + (size_t)side * 5 * NPT + pt;
-      const double sg = (flip == 0) ? lh : -lh;
-#pragma unroll
-      for (int v = 0; v < 5; ++v) ut[v] += sg * F[v * NPT];
-    }
-  }
-  // Ut = -Ut*sJ  (+ source)
-  const double sj = P.sJ[(size_t)e * NP3 + t];
-  const double tStage = P.dtDev ? (P.dtDev[1] + P.rkC * P.dtDev[0]) : P.t;
-#pragma unroll
-  for (int v = 0; v < 5; ++v) ut[v] = ut[v] * (-sj);
-  if (P.source) {  // CalcSource CASE(4), equation.f90:1000-1024
-    const double* x = P.xGP + 3 * ((size_t)e * NP3 + t);
-    double arg = P.srcOmega * (x[0] + x[1] + x[2] - tStage);
-    double c = cos(arg), sn = sin(arg), s2 = 2. * sn * c;
-    ut[0] += P.srcTmp[0] * c;
-    double mm = P.srcTmp[1] * c + P.srcTmp[2] * s2;
-    ut[1] += mm; ut[2] += mm; ut[3] += mm;
-    ut[4] += P.srcTmp[3] * c + P.srcTmp[4] * s2 + P.srcTmp[5] * sn;
-  }
-  const size_t o = 5 * ((size_t)e * NP3 + t);
-  if (P.stage == 0) {
-#pragma unroll
-    for (int v = 0; v < 5; ++v) P.Ut[o + v] = ut[v];
+  for (int v = 0; v < 5; ++v) ut[v] = acc[vol_pad<NP, LPW>(t) * 5 + v];
+  vol_finish_node<NP, VISC>(P, e, t, u, ut, sE2S[eb]);
+}
+
+// ------------------------------------------------------------------------------------------------
+// Volume kernel for even N+1 in {4, 6, 8}: the same sums as volume_kernel with two nodes of a line per
+// thread.  The one-node form waits on shared loads, shuffles and the chain of one pair flux at a time (FP64
+// pipe 46 % busy at N = 7): a pair takes ~20 shared loads and 10 32-bit shuffles there.  Here thread I of
+// the G = (N+1)/2 threads of a line holds nodes I and I+G in registers and meets the other threads' two
+// nodes at a time: its own pair first, then in round r = 1..(G-1)/2 the four pairs with the nodes of
+// thread I+r, and for even G a last round shared between the two threads of each opposite couple, two
+// pairs each.  A partner node's record is loaded once for two pairs and its sum shuffled back once, no
+// lane idles in a half-filled round, and the pairs are evaluated two at a time (pair_flux2).  One thread handles two nodes in the prologue
+// and epilogue as well; the metrics go to the records by asynchronous copies while the node's
+// quantities are formed (the pair fluxes that average two half metrics take whole ones and the
+// operator scaled by 1/2: exact).
+//
+// Measured, one B200, one-node form -> this one: Navier-Stokes N = 5 right-hand side (BR2, 463 k nodes) 228 ->
+// 204 us, N = 7 step (32^3 elements) 23.2 -> 22.7 ms, Euler N = 3 with subcells (512 k nodes, two steps) 1570 ->
+// 1486 us.  What bounds it now is latency again: 16 warps per SM at 128 registers, issue slots a third
+// busy, most stalls on the FP64 results of the own chain.  Where a mesh has too few elements to fill the
+// SMs (Euler N = 3, 512 elements) the one-node form's shorter chain per thread wins, so it stays among the
+// candidates of the launch-shape tuning (vol_shapes.h).
+//
+// Node slots (vb_slot) make every half-warp's 8-byte record and accumulator accesses hit 16 distinct
+// bank pairs, in the pair phase of all three directions and in the node phases: for N+1 = 8 and 4 a
+// permutation of the nodes whose low four bits differ over (position of thread I, lines of the
+// half-warp); the lines are dealt to warps in the order of vb_line.
+// ------------------------------------------------------------------------------------------------
+template <int NP>
+__host__ __device__ constexpr int vb_slot(int i, int j, int k) {
+  if (NP == 8)
+    return ((i ^ j) & 3) | (((k ^ (i >> 2)) & 1) << 2) | ((((k >> 1) ^ j) & 1) << 3) | (j << 4) | ((k >> 2) << 7) |
+           ((i >> 2) << 8);
+  if (NP == 4) return (i + 4 * j + 16 * k) ^ ((k & 1) << 1) ^ ((k >> 1) << 3);
+  return i + NP * j + (NP * NP + 1) * k;
+}
+template <int NP>
+__host__ __device__ constexpr int vb_slots() { return NP == 6 ? 221 : NP * NP * NP; }
+
+// coordinates (a, b) of line `ln` of direction `dir` (dir 0: j, k; 1: i, k; 2: i, j)
+template <int NP>
+__device__ __forceinline__ void vb_line(int dir, int ln, int& a, int& b) {
+  if (NP == 8) {
+    if (dir == 2) { a = ln & 7; b = ln >> 3; }               // i varies fastest
+    else { b = (ln & 3) | ((ln >> 5) << 2); a = (ln >> 2) & 7; }  // the low bits of k vary fastest
+  } else if (NP == 4) {
+    if (dir == 0) { a = ln & 3; b = ln >> 2; }
+    else if (dir == 1) { a = ln & 3; b = (ln >> 3) | (((ln >> 2) & 1) << 1); }
+    else { a = (ln & 1) | ((ln >> 3) << 1); b = (ln >> 1) & 3; }
   } else {
-    // LSERK-2reg stage: Ut_tmp = Ut - A*Ut_tmp (stage 1: Ut_tmp = Ut); U = U + b*dt*Ut_tmp
-    const double dt = stage_dt(P, e);
-    const double bdt = P.rkB * dt;
+    a = ln % NP; b = ln / NP;
+  }
+}
+
+template <int NP, int EPB>
+struct VolBlkShape {
+  static constexpr int G = NP / 2, LPW = 32 / G, WARPS = (EPB * NP * NP + LPW - 1) / LPW, THREADS = 32 * WARPS;
+};
+
+template <int NP, int VF, int EPB>
+__host__ __device__ constexpr size_t vol_blk_smem_bytes() {
+  return sizeof(double) * (size_t)(NP * NP + EPB * (VolRec<VF>::RS + 5) * vb_slots<NP>());
+}
+
+__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+template <int NP, int VF, bool VISC, int EPB, int MINB>
+__global__ void __launch_bounds__(VolBlkShape<NP, EPB>::THREADS, MINB) volume_blk_kernel(KParams P) {
+  if (halted(P)) return;
+  using SH = VolBlkShape<NP, EPB>;
+  constexpr int NP3 = NP * NP * NP, NPT = NP * NP, G = SH::G, LPW = SH::LPW, NS = vb_slots<NP>();
+  constexpr int RS = VolRec<VF>::RS, NF = VolRec<VF>::NF, MO = VolRec<VF>::MO, NODES = EPB * NP3;
+  constexpr int IT = (NODES + SH::THREADS - 1) / SH::THREADS;
+  static_assert(NP % 2 == 0 && NP >= 4, "two nodes per thread");
+  extern __shared__ double smem[];
+  double* sDvs = smem;          // Dvolsurf(i,l) at [i*NP+l] (x 1/2 where the flux averages the metric)
+  double* recs = sDvs + NPT;    // [element][slot][RS], then the accumulators [element][slot][5]
+  double* accs = recs + (size_t)EPB * NS * RS;
+  __shared__ int sE2S[EPB][12];  // the elements' ElemToSide (side, flip per local side)
+  const int e0 = blockIdx.x * EPB;
+  const int ne = P.nElems - e0 < EPB ? P.nElems - e0 : EPB;
+  for (int z = threadIdx.x; z < NPT; z += SH::THREADS) sDvs[z] = (VF == 0 ? 1.0 : 0.5) * P.basis->Dvs[z];
+  for (int z = threadIdx.x; z < 12 * ne; z += SH::THREADS) sE2S[z / 12][z % 12] = P.e2s[12 * (size_t)e0 + z];
+  if (P.pfTiles > 0 && threadIdx.x == 0) {  // the tile one wave ahead: its inputs into L2
+    const size_t en = ((size_t)blockIdx.x + P.pfTiles) * EPB;
+    if (en < (size_t)P.nElems) {
+      const size_t nn = ((size_t)P.nElems - en < (size_t)EPB ? (size_t)P.nElems - en : (size_t)EPB) * NP3;
+      prefetch_l2_bulk(P.U + 5 * en * NP3, 5 * nn * sizeof(double));
+      prefetch_l2_bulk(P.metrics + 9 * en * NP3, 9 * nn * sizeof(double));
+      prefetch_l2_bulk(P.sJ + en * NP3, nn * sizeof(double));
+      if (VISC) prefetch_l2_bulk(P.utvisc + 4 * en * NP3, 4 * nn * sizeof(double));
+      if (P.stage > 1) prefetch_l2_bulk(P.UtTmp + 5 * en * NP3, 5 * nn * sizeof(double));
+    }
+  }
+  // records: metrics by asynchronous copies, then the flux quantities
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    const int n = threadIdx.x + it * SH::THREADS, el = n / NP3, t = n - el * NP3;
+    if (el < ne) {
+      double* r = recs + ((size_t)el * NS + vb_slot<NP>(t % NP, (t / NP) % NP, t / NPT)) * RS + MO;
+      const double* Mg = P.metrics + (size_t)(e0 + el) * 9 * NP3 + t;
+#pragma unroll
+      for (int c = 0; c < 9; ++c) cp_async8(r + c, Mg + c * NP3);
+    }
+  }
+  {
+    double u[IT][5];
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+      const int n = threadIdx.x + it * SH::THREADS;
+      if (n / NP3 < ne) {
+        const double* Ug = P.U + 5 * ((size_t)e0 * NP3 + n);
+#pragma unroll
+        for (int v = 0; v < 5; ++v) u[it][v] = Ug[v];
+        // the epilogue's operands are needed only after the pair loops: start their way to L2 now
+        prefetch_l2(P.sJ + (size_t)e0 * NP3 + n);
+        if (P.stage > 1) prefetch_l2(P.UtTmp + 5 * ((size_t)e0 * NP3 + n));
+        if constexpr (VISC) {
+          const int el = n / NP3, t = n - el * NP3;
+#pragma unroll
+          for (int v = 0; v < 4; ++v) prefetch_l2(P.utvisc + (size_t)(e0 + el) * 4 * NP3 + v * NP3 + t);
+        }
+      }
+    }
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+      const int n = threadIdx.x + it * SH::THREADS, el = n / NP3, t = n - el * NP3;
+      if (el < ne)
+        make_record<VF>(P, u[it], recs + ((size_t)el * NS + vb_slot<NP>(t % NP, (t / NP) % NP, t / NPT)) * RS);
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  // split-form volume integral, line by line
+  {
+    const int lane = threadIdx.x & 31, ls = lane / G, I = lane - ls * G;
+    const int gl = (threadIdx.x >> 5) * LPW + ls;
+    // lv: this thread's line exists (idle threads keep in-range indexes and only join the shuffles)
+    const bool lv = ls < LPW && gl < ne * NPT;
+    const int pe = lv ? gl / NPT : 0, Ln = lv ? gl - pe * NPT : 0;
+    const double* rec = recs + (size_t)pe * NS * RS;
+    double* acc = accs + (size_t)pe * NS * 5;
+    const int lbase = ls * G;
+#pragma unroll 1
+    for (int dir = 0; dir < 3; ++dir) {
+      int la, lb;
+      vb_line<NP>(dir, Ln, la, lb);
+      auto slot = [&](int x) {
+        return dir == 0 ? vb_slot<NP>(x, la, lb) : (dir == 1 ? vb_slot<NP>(la, x, lb) : vb_slot<NP>(la, lb, x));
+      };
+      const int x0 = I, x1 = I + G;
+      const int s0 = slot(x0), s1 = slot(x1);
+      const double *r0 = rec + s0 * RS, *r1 = rec + s1 * RS;
+      double q0[NF], q1[NF], m0[3], m1[3], a0[5], a1[5];
+      load_rec<VF>(r0, q0);
+      load_rec<VF>(r1, q1);
+      load_metric<VF>(r0, dir, m0);
+      load_metric<VF>(r1, dir, m1);
+      {  // the thread's own pair
+        double F[5];
+        pair_flux<VF>(P, q0, q1, r0, r1, m0, m1, F);
+        const double d0 = sDvs[x0 * NP + x1], d1 = sDvs[x1 * NP + x0];
+#pragma unroll
+        for (int v = 0; v < 5; ++v) { a0[v] = d0 * F[v]; a1[v] = d1 * F[v]; }
+      }
+#pragma unroll
+      for (int r = 1; r <= (G - 1) / 2; ++r) {  // both own nodes with both nodes of thread I + r
+        const int J = I + r < G ? I + r : I + r - G, from = I - r < 0 ? I - r + G : I - r;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int y = J + h * G;
+          const double* ry = rec + slot(y) * RS;
+          double qy[NF], my[3], F[5], G0[5], b[5];
+          load_rec<VF>(ry, qy);
+          load_metric<VF>(ry, dir, my);
+          pair_flux2<VF>(P, q0, qy, r0, ry, m0, my, q1, qy, r1, ry, m1, my, F, G0);
+          const double d0 = sDvs[x0 * NP + y], e0_ = sDvs[y * NP + x0], d1 = sDvs[x1 * NP + y], e1_ = sDvs[y * NP + x1];
+#pragma unroll
+          for (int v = 0; v < 5; ++v) {
+            a0[v] = fma(d0, F[v], a0[v]);
+            a1[v] = fma(d1, G0[v], a1[v]);
+            b[v] = fma(e1_, G0[v], e0_ * F[v]);
+          }
+#pragma unroll
+          for (int v = 0; v < 5; ++v) {
+            const double got = __shfl_sync(0xffffffffu, b[v], (lbase + from) & 31);
+            if (h == 0) a0[v] += got;
+            else a1[v] += got;
+          }
+        }
+      }
+      if constexpr (G % 2 == 0) {
+        // opposite threads: the lower takes (own 0, other 0) and (own 1, other 1), the upper (own 0,
+        // other 1) and (own 1, other 0)
+        const bool up = I >= G / 2;
+        const int J = up ? I - G / 2 : I + G / 2;
+        const int y0 = up ? J + G : J, y1 = up ? J : J + G;  // partners of own 0 and own 1
+        const double *ra = rec + slot(y0) * RS, *rb = rec + slot(y1) * RS;
+        double qa[NF], ma[3], qb[NF], mb[3], F[5], H[5];
+        load_rec<VF>(ra, qa);
+        load_metric<VF>(ra, dir, ma);
+        load_rec<VF>(rb, qb);
+        load_metric<VF>(rb, dir, mb);
+        pair_flux2<VF>(P, q0, qa, r0, ra, m0, ma, q1, qb, r1, rb, m1, mb, F, H);
+        const double d0 = sDvs[x0 * NP + y0], d1 = sDvs[x1 * NP + y1];
+        const double e0_ = sDvs[y0 * NP + x0], e1_ = sDvs[y1 * NP + x1];
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+          a0[v] = fma(d0, F[v], a0[v]);
+          a1[v] = fma(d1, H[v], a1[v]);
+          // the share of the other thread's node 0, then of its node 1
+          const double b0 = e0_ * F[v], b1 = e1_ * H[v];
+          a0[v] += __shfl_sync(0xffffffffu, up ? b1 : b0, (lbase + J) & 31);
+          a1[v] += __shfl_sync(0xffffffffu, up ? b0 : b1, (lbase + J) & 31);
+        }
+      }
+      if (lv) {
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+          if (dir == 0) {
+            acc[s0 * 5 + v] = a0[v];
+            acc[s1 * 5 + v] = a1[v];
+          } else {
+            acc[s0 * 5 + v] += a0[v];
+            acc[s1 * 5 + v] += a1[v];
+          }
+        }
+      }
+      __syncthreads();
+    }
+  }
+#pragma unroll 1
+  for (int it = 0; it < IT; ++it) {
+    const int n = threadIdx.x + it * SH::THREADS, el = n / NP3, t = n - el * NP3;
+    if (el >= ne) break;
+    const double* Ug = P.U + 5 * ((size_t)e0 * NP3 + n);
+    const double* ac = accs + ((size_t)el * NS + vb_slot<NP>(t % NP, (t / NP) % NP, t / NPT)) * 5;
+    double u[5], ut[5];
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-      double tmp = (P.stage == 1) ? ut[v] : ut[v] - P.UtTmp[o + v] * P.rkA;
-      P.UtTmp[o + v] = tmp;
-      P.U[o + v] = u[v] + tmp * bdt;
+      u[v] = Ug[v];
+      ut[v] = ac[v];
     }
+    vol_finish_node<NP, VISC>(P, e0 + el, t, u, ut, sE2S[el]);
   }
 }
 

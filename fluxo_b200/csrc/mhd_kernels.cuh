@@ -149,10 +149,38 @@ __device__ __forceinline__ void make_rec(const KParams& P, const double* U, doub
   }
 }
 
-// F = F#(L, R; metrics), symmetric in (L, R)
+// Log means of a pair (as for the Euler fluxes, volume_pairs.cuh): mn[0] = LN(rho), mn[1] = 1/LN of beta
+// (Derigs) or of the internal energy (FloGor), entry B of the record, mn[2] = 1/(B_L + B_R)
+template <int VF> struct Means { static constexpr bool USED = false; static constexpr int B = 0, LA = 0, LB = 0; };
+template <> struct Means<10> { static constexpr bool USED = true; static constexpr int B = 1, LA = 12, LB = 13; };
+template <> struct Means<12> { static constexpr bool USED = true; static constexpr int B = 2, LA = 10, LB = 11; };
+
+template <int VF>
+__device__ __forceinline__ bool pair_means(const double* L, const double* R, double* mn) {
+  using M = Means<VF>;
+  if constexpr (!M::USED) return true;
+  else {
+    const double sa = L[0] + R[0], sb = L[M::B] + R[M::B], inv = rcp_nr(sa * sb);
+    mn[2] = sa * inv;
+    return ln_pair(L[0], R[0], sa, sb * inv, L[M::B], R[M::B], mn[2], mn[0], mn[1]);
+  }
+}
+template <int VF>
+__device__ __forceinline__ void pair_means_fix(const double* L, const double* R, const double* lL, const double* lR,
+                                               double* mn) {
+  using M = Means<VF>;
+  if constexpr (M::USED)
+    ln_pair_fix(L[0], R[0], lL + M::LA, lR + M::LA, L[M::B], R[M::B], lL + M::LB, lR + M::LB, mn[0], mn[1]);
+}
+
+// F = F#(L, R; metrics), symmetric in (L, R); lL, lR are the nodes' records (read for their logarithms
+// only, off the log means' series branch)
 template <int VF>
 __device__ __forceinline__ void pair_flux_mhd(const KParams& P, double ch, const double* L, const double* R,
-                                          const double* mL, const double* mR, double* F) {
+                                              const double* lL, const double* lR, const double* mL,
+                                              const double* mR, double* F) {
+  double mn[3];
+  if (!pair_means<VF>(L, R, mn)) pair_means_fix<VF>(L, R, lL, lR, mn);
   const double smu0 = P.smu_0;
   if constexpr (VF == 0) {  // StandardDGFluxVec :492-567
     const double qvL = L[6] * mL[0] + L[7] * mL[1] + L[8] * mL[2], qbL = L[9] * mL[0] + L[10] * mL[1] + L[11] * mL[2];
@@ -186,12 +214,8 @@ __device__ __forceinline__ void pair_flux_mhd(const KParams& P, double ch, const
       for (int d = 0; d < 3; ++d) F[5 + d] = F[5 + d] + phiHat * m[d];
       F[8] = 0.5 * ch * (qbL + qbR);
     } else if constexpr (VF == 10) {  // EntropyAndKinEnergyConservingFluxVec_Derigs :761-848
-      const double sr = L[0] + R[0], sb = L[1] + R[1];
-      const double inv = rcp_nr(sr * sb);
-      const double isr = sb * inv, isb = sr * inv;          // 1/sr, 1/sb
-      const double rhoLN = ln_mean(L, R, 0, 12, sr, isr);   // LN(rho)
-      const double sbLN = inv_ln_mean(L, R, 1, 13, isb);    // 1/LN(beta)
-      const double rsb = sr * isb;                          // (rho_L+rho_R)/(beta_L+beta_R)
+      const double rhoLN = mn[0], sbLN = mn[1];        // LN(rho), 1/LN(beta)
+      const double rsb = (L[0] + R[0]) * mn[2];        // (rho_L+rho_R)/(beta_L+beta_R)
       double vA[3], BA[3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) { vA[d] = 0.5 * (L[2 + d] + R[2 + d]); BA[d] = 0.5 * (L[5 + d] + R[5 + d]); }
@@ -213,10 +237,8 @@ __device__ __forceinline__ void pair_flux_mhd(const KParams& P, double ch, const
       F[4] = F[0] * 0.5 * (P.sKappaM1 * sbLN - 0.5 * (L[9] + R[9])) + (vA[0] * F[1] + vA[1] * F[2] + vA[2] * F[3]) +
              smu0 * (sB - 0.25 * b2v + 0.5 * (L[11] + R[11]) * Bm + F[8] * psiA - (ch * 0.5) * pB);
     } else if constexpr (VF == 12) {  // EntropyAndKinEnergyConservingFluxVec_FloGor :970-1074
-      const double sr = L[0] + R[0], se = L[2] + R[2];
-      const double inv = rcp_nr(sr * se);
-      const double rhoLN = ln_mean(L, R, 0, 10, sr, se * inv);
-      const double ieT = L[2] * R[2] * inv_ln_mean(L, R, 2, 11, sr * inv);  // e_L e_R / LN(e)
+      const double rhoLN = mn[0];
+      const double ieT = L[2] * R[2] * mn[1];  // e_L e_R / LN(e)
       double vA[3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) vA[d] = 0.5 * (L[3 + d] + R[3 + d]);
@@ -370,7 +392,7 @@ __global__ void __launch_bounds__(vol_threads<NP>(), vol_minb<NP>()) volume_kern
         if (active) {
           // the partner's record is read in place (the log-mean logarithms only when needed)
           const double* rq = prec + mpad<NP>(base + q * stride) * RS;
-          pair_flux_mhd<VF>(P, ch, ro, rq, mo, rq + NQ + 3 * dir, F);
+          pair_flux_mhd<VF>(P, ch, ro, rq, ro, rq, mo, rq + NQ + 3 * dir, F);
         }
         const double dOwn = sDvs[p * NP + q], dPart = sDvs[q * NP + p];
         int src = p - d;

@@ -14,17 +14,23 @@ template <int NP, bool VISC, int I>
 static cudaError_t vol_shape_launch(int nElems, cudaStream_t s, const KParams& P) {
   constexpr VolShapeId sh = kVolShapes[NP][I];
   constexpr int EPB = sh.epb, LPW = sh.lpw, MINB = sh.minb, OWNSM = sh.ownsm;
-  constexpr size_t smem = vol_smem_bytes<NP, VF_ID, EPB, LPW>();
   static std::atomic<unsigned long long> attr{0};
   static std::atomic<int> resident[64];
-  auto k = volume_kernel<NP, VF_ID, VISC, EPB, LPW, MINB, OWNSM>;
-  cudaError_t e = smem_attr_once(k, smem, attr);
-  if (e != cudaSuccess) return e;
-  const int grid = (nElems + EPB - 1) / EPB;
-  KParams Q = P;
-  Q.pfTiles = resident_blocks(k, VolShape<NP, EPB, LPW>::THREADS, smem, resident);
-  k<<<grid, VolShape<NP, EPB, LPW>::THREADS, smem, s>>>(Q);
-  return cudaGetLastError();
+  auto launch = [&](auto k, int threads, size_t smem) {
+    cudaError_t e = smem_attr_once(k, smem, attr);
+    if (e != cudaSuccess) return e;
+    const int grid = (nElems + EPB - 1) / EPB;
+    KParams Q = P;
+    Q.pfTiles = resident_blocks(k, threads, smem, resident);
+    k<<<grid, threads, smem, s>>>(Q);
+    return cudaGetLastError();
+  };
+  if constexpr ((NP == 4 || NP == 6 || NP == 8) && LPW == 64 / NP)  // two nodes per thread
+    return launch(volume_blk_kernel<NP, VF_ID, VISC, EPB, MINB>, VolBlkShape<NP, EPB>::THREADS,
+                  vol_blk_smem_bytes<NP, VF_ID, EPB>());
+  else
+    return launch(volume_kernel<NP, VF_ID, VISC, EPB, LPW, MINB, OWNSM>, VolShape<NP, EPB, LPW>::THREADS,
+                  vol_smem_bytes<NP, VF_ID, EPB, LPW>());
 }
 
 template <int NP, bool VISC>

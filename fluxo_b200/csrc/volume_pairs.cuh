@@ -6,7 +6,7 @@
 // VolumeFluxAverageVec family (src/equation/navierstokes/flux_average.f90); results agree with
 // the reference formulas to roundoff:
 //  - the logarithmic mean LN_MEAN (flux_average.f90:1945-1965) keeps its series branch for
-//    u = ((b-a)/(b+a))^2 < 1e-4, as a product with a series in u (ln_mean, inv_ln_mean), and
+//    u = ((b-a)/(b+a))^2 < 1e-4, as a product with a series in u (ln_series, inv_ln_series), and
 //    otherwise uses (b-a)/(log b - log a) with per-node logarithms;
 //  - the divisions of one pair flux are merged into a single reciprocal (rcp_nr).
 #pragma once
@@ -29,60 +29,73 @@ __device__ __forceinline__ double rcp_nr(double x) {
   return fma(y, e, y);
 }
 
-// Logarithmic mean (LN_MEAN) of a = L[i] and b = R[i] and its reciprocal, given s = a + b and is = 1/s.
-// With u = ((b-a)/s)^2 < 1e-4 the mean is s/2 / (1 + u/3 + u^2/5 + u^3/7); ln_mean multiplies by the
-// series of that reciprocal, 1 - u/3 - 4u^2/45 - 44u^3/945 (the next term is below 1e-17), and
-// inv_ln_mean by the polynomial itself, so neither divides: one reciprocal 1/(s_a s_b) serves both means
-// of a pair.  Off the series branch the mean is (b-a)/(log b - log a); the logarithms log a = L[il],
-// log b = R[il] are read only there (R usually points into shared memory: in smooth flows nearly every
-// pair takes the series branch).
-__device__ __forceinline__ double ln_mean(const double* L, const double* R, int i, int il, double s, double is) {
-  const double d = R[i] - L[i], f = d * is, u = f * f;
-  if (u < 1.0e-4) return s * fma(u, fma(u, fma(u, -22. / 945., -2. / 45.), -1. / 6.), 0.5);
-  return d * rcp_nr(R[il] - L[il]);
+// Logarithmic mean (LN_MEAN) of a and b from s = a + b, and its reciprocal from is = 1/s, on the series
+// branch u = ((b-a)/s)^2 < 1e-4, where the mean is s/2 / (1 + u/3 + u^2/5 + u^3/7): ln_series multiplies by
+// the series of that reciprocal, 1 - u/3 - 4u^2/45 - 44u^3/945 (the next term is below 1e-17), and
+// inv_ln_series by the polynomial itself, so neither divides: one reciprocal 1/(s_a s_b) serves both means
+// of a pair.
+__device__ __forceinline__ double ln_series(double s, double u) {
+  return s * fma(u, fma(u, fma(u, -22. / 945., -2. / 45.), -1. / 6.), 0.5);
 }
-__device__ __forceinline__ double inv_ln_mean(const double* L, const double* R, int i, int il, double is) {
-  const double d = R[i] - L[i], f = d * is, u = f * f;
-  if (u < 1.0e-4) return is * fma(u, fma(u, fma(u, 2. / 7., 2. / 5.), 2. / 3.), 2.);
-  return (R[il] - L[il]) * rcp_nr(d);
+__device__ __forceinline__ double inv_ln_series(double is, double u) {
+  return is * fma(u, fma(u, fma(u, 2. / 7., 2. / 5.), 2. / 3.), 2.);
+}
+// The two means of a pair: M = LN(a) and I = 1 / LN(b).  ln_pair forms both by their series and tells whether
+// both are on that branch; ln_pair_fix replaces those that are not by (b-a)/(log b - log a), with the
+// logarithms of the nodes' records (read only here: in smooth flows nearly every pair is on the series
+// branch).  Two steps, so that several pairs share one rare branch and their straight-line parts overlap.
+__device__ __forceinline__ bool ln_pair(double La, double Ra, double sa, double isa, double Lb, double Rb, double isb,
+                                        double& M, double& I) {
+  const double fa = (Ra - La) * isa, fb = (Rb - Lb) * isb;
+  const double ua = fa * fa, ub = fb * fb;
+  M = ln_series(sa, ua);
+  I = inv_ln_series(isb, ub);
+  return ua < 1.0e-4 && ub < 1.0e-4;
+}
+__device__ __forceinline__ void ln_pair_fix(double La, double Ra, const double* lLa, const double* lRa, double Lb,
+                                            double Rb, const double* lLb, const double* lRb, double& M, double& I) {
+  const double da = Ra - La, sa = La + Ra, db = Rb - Lb, sb = Lb + Rb;
+  if (!(da * da < 1.0e-4 * (sa * sa))) M = da * rcp_nr(*lRa - *lLa);
+  if (!(db * db < 1.0e-4 * (sb * sb))) I = (*lRb - *lLb) * rcp_nr(db);
 }
 
-// Record of a node in shared memory: NQ flux quantities at [0, NQ), the metric terms Ja^1..Ja^3
+// Record of a node in shared memory: NQ flux quantities at [0, NQ) (the first NF without
+// the logarithms, which come last), the metric terms Ja^1..Ja^3
 // (x,y,z each) at [MO, MO+9), RS doubles per node.  The odd stride RS spreads the records of the
 // nodes of a line over the shared-memory banks (padded 16-byte-aligned records read with 16-byte
 // loads measured 19 % slower on the N=7 volume kernel).
 template <int VF>
 struct VolRec;
 // standard DG (0) and dealiased metric (1): rho, rho u, rho v, rho w, rho E, u, v, w, p
-template <> struct VolRec<0> { static constexpr int NQ = 9, MO = 9, RS = 19; };
-template <> struct VolRec<1> { static constexpr int NQ = 9, MO = 9, RS = 19; };
+template <> struct VolRec<0> { static constexpr int NQ = 9, NF = 9, MO = 9, RS = 19; };
+template <> struct VolRec<1> { static constexpr int NQ = 9, NF = 9, MO = 9, RS = 19; };
 // Kennedy-Gruber (2): rho, u, v, w, p, e = E/rho
-template <> struct VolRec<2> { static constexpr int NQ = 6, MO = 6, RS = 15; };
+template <> struct VolRec<2> { static constexpr int NQ = 6, NF = 6, MO = 6, RS = 15; };
 // Ducros (3): halves of rho, u, v, w, p, rho u, rho v, rho w, rho E (every average is arithmetic)
-template <> struct VolRec<3> { static constexpr int NQ = 9, MO = 9, RS = 19; };
+template <> struct VolRec<3> { static constexpr int NQ = 9, NF = 9, MO = 9, RS = 19; };
 // Morinishi (4): rho, u, v, w, p, |v|^2
-template <> struct VolRec<4> { static constexpr int NQ = 6, MO = 6, RS = 15; };
+template <> struct VolRec<4> { static constexpr int NQ = 6, NF = 6, MO = 6, RS = 15; };
 // EC-KEP (5): rho, u/2, v/2, w/2, beta = rho/(2p), |v|^2/2, log rho, log beta (the halves make the
 // pair averages plain sums; halving is exact, so the averages are bit-identical)
-template <> struct VolRec<5> { static constexpr int NQ = 8, MO = 8, RS = 17; };
+template <> struct VolRec<5> { static constexpr int NQ = 8, NF = 6, MO = 8, RS = 17; };
 // approximate EC-KEP (6): rho/2, u/2, v/2, w/2, beta, |v|^2/2
-template <> struct VolRec<6> { static constexpr int NQ = 6, MO = 6, RS = 15; };
+template <> struct VolRec<6> { static constexpr int NQ = 6, NF = 6, MO = 6, RS = 15; };
 // EC-KEP with pressure average (7): rho/2, u/2, v/2, w/2, p/2, beta, |v|^2/2, log beta
-template <> struct VolRec<7> { static constexpr int NQ = 8, MO = 8, RS = 17; };
+template <> struct VolRec<7> { static constexpr int NQ = 8, NF = 7, MO = 8, RS = 17; };
 // Kennedy-Gruber, Pirozzoli form (8): halves of rho, u, v, w, p, H = (rho E + p)/rho
-template <> struct VolRec<8> { static constexpr int NQ = 6, MO = 6, RS = 15; };
+template <> struct VolRec<8> { static constexpr int NQ = 6, NF = 6, MO = 6, RS = 15; };
 // Gassner-Winters-Walch (9): halves of sqrt(rho) times (1, u, v, w, H)
-template <> struct VolRec<9> { static constexpr int NQ = 5, MO = 5, RS = 15; };
+template <> struct VolRec<9> { static constexpr int NQ = 5, NF = 5, MO = 5, RS = 15; };
 // Ismail-Roe (10): z1 = sqrt(rho/p), u, v, w, z5 = z1 p, log z1, log z5
-template <> struct VolRec<10> { static constexpr int NQ = 7, MO = 7, RS = 17; };
+template <> struct VolRec<10> { static constexpr int NQ = 7, NF = 5, MO = 7, RS = 17; };
 // Ranocha (32): rho, u, v, w, p, rho/p, log rho, log(rho/p)
-template <> struct VolRec<32> { static constexpr int NQ = 8, MO = 8, RS = 17; };
+template <> struct VolRec<32> { static constexpr int NQ = 8, NF = 6, MO = 8, RS = 17; };
 
-// the NQ flux quantities of record r (shared memory)
+// the flux quantities of record r (shared memory) without the trailing logarithms
 template <int VF>
 __device__ __forceinline__ void load_rec(const double* r, double* q) {
 #pragma unroll
-  for (int z = 0; z < VolRec<VF>::NQ; ++z) q[z] = r[z];
+  for (int z = 0; z < VolRec<VF>::NF; ++z) q[z] = r[z];
 }
 
 // the metric triple Ja^(dir+1) of record r
@@ -135,10 +148,44 @@ __device__ __forceinline__ void make_record(const KParams& P, const double* U, d
   }
 }
 
-// F = F#(L, R) . metric, symmetric in (L, R)
+// Entries of a record that take a log mean (A, logarithm LA) and the reciprocal of one (B, LB)
+template <int VF> struct VolMeans { static constexpr bool USED = false; static constexpr int A = 0, LA = 0, B = 0, LB = 0; };
+template <> struct VolMeans<5> { static constexpr bool USED = true; static constexpr int A = 0, LA = 6, B = 4, LB = 7; };
+template <> struct VolMeans<7> { static constexpr bool USED = true; static constexpr int A = 5, LA = 7, B = 5, LB = 7; };
+template <> struct VolMeans<10> { static constexpr bool USED = true; static constexpr int A = 4, LA = 6, B = 0, LB = 5; };
+template <> struct VolMeans<32> { static constexpr bool USED = true; static constexpr int A = 0, LA = 6, B = 5, LB = 7; };
+
+// The means of a pair's flux: mn[0] = LN(A), mn[1] = 1/LN(B) on the series branch (returns whether both
+// are on it), mn[2] = 1/(B_L + B_R)
 template <int VF>
-__device__ __forceinline__ void pair_flux(const KParams& P, const double* L, const double* R, const double* mL,
-                                          const double* mR, double* F) {
+__device__ __forceinline__ bool pair_means(const double* L, const double* R, double* mn) {
+  using V = VolMeans<VF>;
+  if constexpr (!V::USED) return true;
+  else {
+    const double sa = L[V::A] + R[V::A], sb = L[V::B] + R[V::B];
+    double isa;
+    if constexpr (V::A == V::B) isa = mn[2] = rcp_nr(sa);
+    else {
+      const double inv = rcp_nr(sa * sb);
+      isa = sb * inv;
+      mn[2] = sa * inv;
+    }
+    return ln_pair(L[V::A], R[V::A], sa, isa, L[V::B], R[V::B], mn[2], mn[0], mn[1]);
+  }
+}
+// off the series branch: lL, lR are the nodes' records, read for their logarithms
+template <int VF>
+__device__ __forceinline__ void pair_means_fix(const double* L, const double* R, const double* lL, const double* lR,
+                                               double* mn) {
+  using V = VolMeans<VF>;
+  if constexpr (V::USED)
+    ln_pair_fix(L[V::A], R[V::A], lL + V::LA, lR + V::LA, L[V::B], R[V::B], lL + V::LB, lR + V::LB, mn[0], mn[1]);
+}
+
+// F = F#(L, R) . metric, symmetric in (L, R), from the pair's means mn
+template <int VF>
+__device__ __forceinline__ void pair_flux_from(const KParams& P, const double* L, const double* R, const double* mn,
+                                               const double* mL, const double* mR, double* F) {
   if constexpr (VF == 0) {  // StandardDGFluxVec :394-439
     const double qL = L[5] * mL[0] + L[6] * mL[1] + L[7] * mL[2];
     const double qR = R[5] * mR[0] + R[6] * mR[1] + R[7] * mR[2];
@@ -202,7 +249,7 @@ __device__ __forceinline__ void pair_flux(const KParams& P, const double* L, con
       F[3] = F[0] * wH + m3 * p1;
       F[4] = F[0] * 0.5 * (P.sKappaM1 * sbM - (L[5] + R[5])) + uH * F[1] + vH * F[2] + wH * F[3];
     } else if constexpr (VF == 7) {  // ggFluxVec :1575-1653 (halves)
-      const double sbHat = inv_ln_mean(L, R, 5, 7, rcp_nr(L[5] + R[5]));
+      const double sbHat = mn[1];
       const double rhoM = L[0] + R[0];
       const double uH = L[1] + R[1], vH = L[2] + R[2], wH = L[3] + R[3];
       const double p1 = L[4] + R[4];
@@ -233,12 +280,8 @@ __device__ __forceinline__ void pair_flux(const KParams& P, const double* L, con
       F[3] = q * wH + m3 * p1;
       F[4] = q * HH;
     } else if constexpr (VF == 5) {  // EntropyAndEnergyConservingFluxVec :1277-1356
-      const double sr = L[0] + R[0], sb = L[4] + R[4];
-      const double inv = rcp_nr(sr * sb);
-      const double isr = sb * inv, isb = sr * inv;            // 1/sr, 1/sb
-      const double rhoHat = ln_mean(L, R, 0, 6, sr, isr);     // LN(rho)
-      const double sbHat = inv_ln_mean(L, R, 4, 7, isb);      // 1/LN(beta)
-      const double p1 = 0.5 * sr * isb;                       // 0.5*rho_mean/beta_mean
+      const double rhoHat = mn[0], sbHat = mn[1];        // LN(rho), 1/LN(beta)
+      const double p1 = 0.5 * (L[0] + R[0]) * mn[2];     // 0.5*rho_mean/beta_mean
       const double uH = L[1] + R[1], vH = L[2] + R[2], wH = L[3] + R[3];  // records hold u/2, v/2, w/2
       const double q = uH * m1 + vH * m2 + wH * m3;
       F[0] = rhoHat * q;
@@ -247,16 +290,13 @@ __device__ __forceinline__ void pair_flux(const KParams& P, const double* L, con
       F[3] = F[0] * wH + m3 * p1;
       F[4] = F[0] * 0.5 * (P.sKappaM1 * sbHat - (L[5] + R[5])) + uH * F[1] + vH * F[2] + wH * F[3];
     } else if constexpr (VF == 10) {  // TwoPointEntropyConservingFluxVec :574-673
-      const double s1 = L[0] + R[0], s5 = L[4] + R[4];
-      const double inv = rcp_nr(s1 * s5);
-      const double is1 = s5 * inv, is5 = s1 * inv;               // 1/s1, 1/s5
-      const double z5LN = ln_mean(L, R, 4, 6, s5, is5);
-      const double ratio = z5LN * inv_ln_mean(L, R, 0, 5, is1);  // z5LN / z1LN
-      const double rhoHat = 0.5 * s1 * z5LN;
+      const double z5LN = mn[0], is1 = mn[2];  // is1 = 1/(z1_L + z1_R)
+      const double ratio = z5LN * mn[1];       // z5LN / z1LN
+      const double rhoHat = 0.5 * (L[0] + R[0]) * z5LN;
       const double uH = (L[0] * L[1] + R[0] * R[1]) * is1;
       const double vH = (L[0] * L[2] + R[0] * R[2]) * is1;
       const double wH = (L[0] * L[3] + R[0] * R[3]) * is1;
-      const double p1 = s5 * is1;
+      const double p1 = (L[4] + R[4]) * is1;
       const double q = uH * m1 + vH * m2 + wH * m3;
       F[0] = rhoHat * q;
       F[1] = F[0] * uH + m1 * p1;
@@ -264,10 +304,7 @@ __device__ __forceinline__ void pair_flux(const KParams& P, const double* L, con
       F[3] = F[0] * wH + m3 * p1;
       F[4] = 0.5 * (q * P.kappaP1 * P.sKappaM1 * ratio + uH * F[1] + vH * F[2] + wH * F[3]);
     } else if constexpr (VF == 32) {  // RanochaFluxVec :1876-1929
-      const double sr = L[0] + R[0], ss = L[5] + R[5];
-      const double inv = rcp_nr(sr * ss);
-      const double rhoLN = ln_mean(L, R, 0, 6, sr, ss * inv);
-      const double srspM = inv_ln_mean(L, R, 5, 7, sr * inv);  // 1/LN(rho/p)
+      const double rhoLN = mn[0], srspM = mn[1];  // LN(rho), 1/LN(rho/p)
       const double va1 = 0.5 * (L[1] + R[1]), va2 = 0.5 * (L[2] + R[2]), va3 = 0.5 * (L[3] + R[3]);
       const double v2zip = 0.5 * (L[1] * R[1] + L[2] * R[2] + L[3] * R[3]);
       const double pavg = 0.5 * (L[4] + R[4]);
@@ -280,6 +317,31 @@ __device__ __forceinline__ void pair_flux(const KParams& P, const double* L, con
       F[4] = F[0] * (v2zip + srspM * P.sKappaM1) + 0.5 * (L[4] * vmR + R[4] * vmL);
     }
   }
+}
+
+// the flux of one pair; lL, lR are the nodes' records (L and R may be copies without the logarithms)
+template <int VF>
+__device__ __forceinline__ void pair_flux(const KParams& P, const double* L, const double* R, const double* lL,
+                                          const double* lR, const double* mL, const double* mR, double* F) {
+  double mn[3];
+  if (!pair_means<VF>(L, R, mn)) pair_means_fix<VF>(L, R, lL, lR, mn);
+  pair_flux_from<VF>(P, L, R, mn, mL, mR, F);
+}
+
+// The fluxes F and H of the pairs (x0, y0) and (x1, y1), side by side: one branch off the series for both
+template <int VF>
+__device__ __forceinline__ void pair_flux2(const KParams& P, const double* x0, const double* y0, const double* l0,
+                                           const double* k0, const double* m0, const double* n0, const double* x1,
+                                           const double* y1, const double* l1, const double* k1, const double* m1,
+                                           const double* n1, double* F, double* H) {
+  double a[3], b[3];
+  const bool sa = pair_means<VF>(x0, y0, a), sb = pair_means<VF>(x1, y1, b);
+  if (!(sa && sb)) {
+    pair_means_fix<VF>(x0, y0, l0, k0, a);
+    pair_means_fix<VF>(x1, y1, l1, k1, b);
+  }
+  pair_flux_from<VF>(P, x0, y0, a, m0, n0, F);
+  pair_flux_from<VF>(P, x1, y1, b, m1, n1, H);
 }
 
 }  // namespace fluxo
