@@ -112,13 +112,14 @@ __global__ void lift_flux_kernel(KParams P, int NP) {
 // ------------------------------------------------------------------------------------------------
 template <int VF> struct Rec;
 // standard DG (0) / dealiased metric (1): rho, rho v(3), E - psi^2/(2mu0), p_t, v(3), B(3), psi, v.B
-// (NQ state entries, then the metrics of the three directions; B, PSI, V: offsets of B, psi, v)
-template <> struct Rec<0> { static constexpr int NQ = 15, RS = 24, B = 9, PSI = 12, V = 6; };
-template <> struct Rec<1> { static constexpr int NQ = 15, RS = 24, B = 9, PSI = 12, V = 6; };
+// (NQ state entries, the first NF without the logarithms or padding, then the metrics of the three
+// directions; B, PSI, V: offsets of B, psi, v)
+template <> struct Rec<0> { static constexpr int NQ = 15, NF = 14, RS = 24, B = 9, PSI = 12, V = 6; };
+template <> struct Rec<1> { static constexpr int NQ = 15, NF = 14, RS = 24, B = 9, PSI = 12, V = 6; };
 // Derigs (10): rho, beta, v(3), B(3), psi, |v|^2, |B|^2, v.B, log rho, log beta
-template <> struct Rec<10> { static constexpr int NQ = 14, RS = 23, B = 5, PSI = 8, V = 2; };
+template <> struct Rec<10> { static constexpr int NQ = 14, NF = 12, RS = 23, B = 5, PSI = 8, V = 2; };
 // FloGor (12): rho, p, e_in, v(3), B(3), psi, log rho, log e_in
-template <> struct Rec<12> { static constexpr int NQ = 12, RS = 21, B = 6, PSI = 9, V = 3; };
+template <> struct Rec<12> { static constexpr int NQ = 12, NF = 10, RS = 21, B = 6, PSI = 9, V = 3; };
 
 constexpr int NACC = NV + 2;  // accumulator per node: Ut (9), non-conservative MHD and GLM line sums
 
@@ -272,8 +273,12 @@ __device__ __forceinline__ void pair_flux_mhd(const KParams& P, double ch, const
 // Jacobian, GLM damping (mhd/equation.f90:1698-1706), optional LSERK stage.
 //
 // The non-conservative term of node i along one line is Phi(i) * sum_l Dvs(i,l) (Bhat_i +
-// (M_i+M_l)/2 . B_l) = Phi(i) * (Bhat_i rowsum_i + M_i/2 . sum_l Dvs B_l + 1/2 sum_l Dvs Bhat_l): four
-// line sums per direction, accumulated over the directions into one scalar per node.
+// (M_i+M_l)/2 . B_l) = Phi(i) * (Bhat_i rowsum_i + sum_l Dvs(i,l) m_il . B_l) with the pair's mean metric
+// m_il, and its GLM part v_i.M_i/2 * (psi_i rowsum_i + sum_l Dvs(i,l) psi_l): two more sums that ride along
+// with the pairs of the line, accumulated over the directions into one scalar each per node.  (The
+// diagonal of Dvs is zero.)  A separate pass over the line for them (8 shared loads per node of the line
+// and 13 multiply-adds) made the resistive N = 4 step on 24^3 elements 7.93 ms; riding along (two more
+// shuffled values per pair) 7.72 ms.
 // ------------------------------------------------------------------------------------------------
 template <int NP>
 __host__ __device__ constexpr int epb() { return (256 / (NP * NP * NP)) > 0 ? (256 / (NP * NP * NP)) : 1; }
@@ -306,143 +311,15 @@ __host__ __device__ constexpr int vol_threads() { return VolShape<NP, epb<NP>(),
 template <int NP>
 __host__ __device__ constexpr int vol_minb() { return vol_threads<NP>() <= 320 ? 2 : 1; }
 
-template <int NP, int VF>
-__global__ void __launch_bounds__(vol_threads<NP>(), vol_minb<NP>()) volume_kernel(KParams P) {
-  if (halted(P)) return;
+// Node epilogue of the volume kernel: from the line sums ut (split form), ncMHD and ncGLM
+// (non-conservative) of node t of element e to Ut (stage 0) or the LSERK update
+template <int NP>
+__device__ __forceinline__ void vol_finish_node(const KParams& P, double ch, int e, int t, const double* u, double* ut,
+                                                double ncMHD, double ncGLM) {
+  constexpr int NP3 = NP * NP * NP, N = NP - 1, NPT = NP * NP;
   const int NC = P.noncons;
   const bool NCGLM = NC != 0 && P.ncGLM != 0;
-  constexpr int NP3 = NP * NP * NP, N = NP - 1, NPT = NP * NP, EPB = epb<NP>(), LPW = vol_lpw<NP>();
-  constexpr int RS = Rec<VF>::RS, NQ = Rec<VF>::NQ, IB = Rec<VF>::B, IPSI = Rec<VF>::PSI, IV = Rec<VF>::V;
-  constexpr int NS = mpad_slots<NP>();
-  extern __shared__ double smem[];
-  double* sDvs = smem;        // Dvolsurf(i,l) at [i*NP+l]
-  double* sRow = sDvs + NPT;  // sum_l Dvolsurf(i,l)
-  // node phases: thread -> (element slot eb, node t); with packed lines the threads past EPB*NP3 idle
-  const bool nodeThread = threadIdx.x < EPB * NP3;
-  const int eb = nodeThread ? threadIdx.x / NP3 : 0, t = nodeThread ? threadIdx.x - eb * NP3 : 0;
-  const int e = blockIdx.x * EPB + eb;
-  const bool valid = nodeThread && e < P.nElems;
-  double* rec = sRow + NP + (size_t)eb * (RS + NACC) * NS;  // [slot][RS]
-  double* acc = rec + (size_t)RS * NS;                       // [slot][NACC]
-  for (int z = threadIdx.x; z < NPT; z += blockDim.x) sDvs[z] = P.basis->Dvs[z];
-  if (threadIdx.x < NP) {
-    double s = 0.;
-    for (int l = 0; l < NP; ++l) s += P.basis->Dvs[threadIdx.x * NP + l];
-    sRow[threadIdx.x] = s;
-  }
-  const double ch = glm_ch(P);
-  double u[NV];
-  if (valid) {
-    const double* Ug = P.U + NV * ((size_t)e * NP3 + t);
-#pragma unroll
-    for (int v = 0; v < NV; ++v) u[v] = Ug[v];
-    prefetch_l2(P.sJ + (size_t)e * NP3 + t);
-    double* r = rec + mpad<NP>(t) * RS;
-    make_rec<VF>(P, u, r);
-    const double* Mg = P.metrics + (size_t)e * 9 * NP3 + t;
-#pragma unroll
-    for (int c = 0; c < 9; ++c) r[NQ + c] = Mg[c * NP3];
-#pragma unroll
-    for (int v = 0; v < NACC; ++v) acc[mpad<NP>(t) * NACC + v] = 0.;
-  }
-  __syncthreads();
-  {
-    // this thread's (element slot pe, line Ln, position p) in the pair phase; lv: it holds a position
-    // of a line of an existing element (idle lanes keep in-range indexes and only join the shuffles)
-    int pe, p, Ln, lbase;
-    bool lv;
-    const int lane = threadIdx.x & 31;
-    if constexpr (LPW == 0) {
-      pe = eb; p = t % NP; Ln = t / NP; lv = valid; lbase = lane - p;
-    } else {
-      constexpr int G = 32 / LPW, WPE = VolShape<NP, EPB, LPW>::WPE;
-      const int wi = threadIdx.x >> 5, slot = lane / G;
-      pe = wi / WPE;
-      p = lane - slot * G;
-      Ln = (wi - pe * WPE) * LPW + slot;
-      lv = slot < LPW && p < NP && Ln < NPT && (int)blockIdx.x * EPB + pe < P.nElems;
-      lbase = slot * G;
-      if (!lv) { p = 0; Ln = 0; }
-    }
-    const int la = Ln % NP, lb = Ln / NP;
-    double* prec = sRow + NP + (size_t)pe * (RS + NACC) * NS;
-    double* pacc = prec + (size_t)RS * NS;
-#pragma unroll 1
-    for (int dir = 0; dir < 3; ++dir) {
-      const int stride = dir == 0 ? 1 : (dir == 1 ? NP : NPT);
-      const int base = dir == 0 ? NP * (la + NP * lb) : (dir == 1 ? la + NPT * lb : la + NP * lb);
-      const int own = base + p * stride, os = mpad<NP>(own);
-      double ro[NQ], mo[3], racc[NV];
-#pragma unroll
-      for (int v = 0; v < NV; ++v) racc[v] = 0.;
-      if (lv) {
-#pragma unroll
-        for (int z = 0; z < NQ; ++z) ro[z] = prec[os * RS + z];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) mo[c] = prec[os * RS + NQ + 3 * dir + c];
-      }
-#pragma unroll
-      for (int d = 1; d <= NP / 2; ++d) {
-        const bool active = lv && (2 * d < NP || p < d);
-        int q = p + d;
-        if (q >= NP) q -= NP;
-        double F[NV];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) F[v] = 0.;
-        if (active) {
-          // the partner's record is read in place (the log-mean logarithms only when needed)
-          const double* rq = prec + mpad<NP>(base + q * stride) * RS;
-          pair_flux_mhd<VF>(P, ch, ro, rq, ro, rq, mo, rq + NQ + 3 * dir, F);
-        }
-        const double dOwn = sDvs[p * NP + q], dPart = sDvs[q * NP + p];
-        int src = p - d;
-        if (src < 0) src += NP;
-        const bool receive = lv && (2 * d < NP || p >= d);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-          racc[v] += active ? dOwn * F[v] : 0.;
-          const double got = __shfl_sync(0xffffffffu, dPart * F[v], (lbase + src) & 31);
-          racc[v] += receive ? got : 0.;
-        }
-      }
-      double ncMHD = 0., ncGLM = 0.;  // this direction's non-conservative line sums of node `own`
-      {
-        if (lv && NC != 0) {
-          double sB0 = 0., sB1 = 0., sB2 = 0., sBh = 0., sPsi = 0.;
-#pragma unroll
-          for (int l = 0; l < NP; ++l) {
-            const double* rl = prec + mpad<NP>(base + l * stride) * RS;
-            const double dl = sDvs[p * NP + l];
-            const double b0 = rl[IB], b1 = rl[IB + 1], b2 = rl[IB + 2];
-            const double* ml = rl + NQ + 3 * dir;
-            sB0 += dl * b0; sB1 += dl * b1; sB2 += dl * b2;
-            sBh += dl * (ml[0] * b0 + ml[1] * b1 + ml[2] * b2);
-            sPsi += dl * rl[IPSI];
-          }
-          const double bhat = mo[0] * ro[IB] + mo[1] * ro[IB + 1] + mo[2] * ro[IB + 2];
-          ncMHD = bhat * sRow[p] + 0.5 * (mo[0] * sB0 + mo[1] * sB1 + mo[2] * sB2) + 0.5 * sBh;
-          if (NCGLM) {
-            const double vm = mo[0] * ro[IV] + mo[1] * ro[IV + 1] + mo[2] * ro[IV + 2];
-            ncGLM = 0.5 * vm * (ro[IPSI] * sRow[p] + sPsi);
-          }
-        }
-      }
-      if (lv) {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) pacc[os * NACC + v] += racc[v];
-        pacc[os * NACC + NV] += ncMHD;
-        pacc[os * NACC + NV + 1] += ncGLM;
-      }
-      __syncthreads();
-    }
-  }
-  double ut[NV];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) ut[v] = valid ? acc[mpad<NP>(t) * NACC + v] : 0.;
-  const double ncMHD = valid ? acc[mpad<NP>(t) * NACC + NV] : 0.;
-  const double ncGLM = valid ? acc[mpad<NP>(t) * NACC + NV + 1] : 0.;
   const int i = t % NP, j = (t / NP) % NP, k = t / NPT;
-  if (!valid) return;
   if (NC != 0) {  // Phi(i) * sum of the line terms (Powell / Brackbill / Janhunen)
     const double srho = 1. / u[0];
     const double v0 = u[1] * srho, v1 = u[2] * srho, v2 = u[3] * srho;
@@ -518,6 +395,128 @@ __global__ void __launch_bounds__(vol_threads<NP>(), vol_minb<NP>()) volume_kern
       P.U[o + v] = u[v] + tmp * bdt;
     }
   }
+}
+
+template <int NP, int VF>
+__global__ void __launch_bounds__(vol_threads<NP>(), vol_minb<NP>()) volume_kernel(KParams P) {
+  if (halted(P)) return;
+  constexpr int NP3 = NP * NP * NP, NPT = NP * NP, EPB = epb<NP>(), LPW = vol_lpw<NP>();
+  constexpr int RS = Rec<VF>::RS, NQ = Rec<VF>::NQ, NF = Rec<VF>::NF, IB = Rec<VF>::B, IPSI = Rec<VF>::PSI, IV = Rec<VF>::V, NE = NV + 2;
+  constexpr int NS = mpad_slots<NP>();
+  extern __shared__ double smem[];
+  double* sDvs = smem;        // Dvolsurf(i,l) at [i*NP+l]
+  double* sRow = sDvs + NPT;  // sum_l Dvolsurf(i,l)
+  // node phases: thread -> (element slot eb, node t); with packed lines the threads past EPB*NP3 idle
+  const bool nodeThread = threadIdx.x < EPB * NP3;
+  const int eb = nodeThread ? threadIdx.x / NP3 : 0, t = nodeThread ? threadIdx.x - eb * NP3 : 0;
+  const int e = blockIdx.x * EPB + eb;
+  const bool valid = nodeThread && e < P.nElems;
+  double* rec = sRow + NP + (size_t)eb * (RS + NACC) * NS;  // [slot][RS]
+  double* acc = rec + (size_t)RS * NS;                       // [slot][NACC]
+  for (int z = threadIdx.x; z < NPT; z += blockDim.x) sDvs[z] = P.basis->Dvs[z];
+  if (threadIdx.x < NP) {
+    double s = 0.;
+    for (int l = 0; l < NP; ++l) s += P.basis->Dvs[threadIdx.x * NP + l];
+    sRow[threadIdx.x] = s;
+  }
+  const double ch = glm_ch(P);
+  double u[NV];
+  if (valid) {
+    const double* Ug = P.U + NV * ((size_t)e * NP3 + t);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) u[v] = Ug[v];
+    prefetch_l2(P.sJ + (size_t)e * NP3 + t);
+    double* r = rec + mpad<NP>(t) * RS;
+    make_rec<VF>(P, u, r);
+    const double* Mg = P.metrics + (size_t)e * 9 * NP3 + t;
+#pragma unroll
+    for (int c = 0; c < 9; ++c) r[NQ + c] = Mg[c * NP3];
+#pragma unroll
+    for (int v = 0; v < NACC; ++v) acc[mpad<NP>(t) * NACC + v] = 0.;
+  }
+  __syncthreads();
+  {
+    // this thread's (element slot pe, line Ln, position p) in the pair phase; lv: it holds a position
+    // of a line of an existing element (idle lanes keep in-range indexes and only join the shuffles)
+    int pe, p, Ln, lbase;
+    bool lv;
+    const int lane = threadIdx.x & 31;
+    if constexpr (LPW == 0) {
+      pe = eb; p = t % NP; Ln = t / NP; lv = valid; lbase = lane - p;
+    } else {
+      constexpr int G = 32 / LPW, WPE = VolShape<NP, EPB, LPW>::WPE;
+      const int wi = threadIdx.x >> 5, slot = lane / G;
+      pe = wi / WPE;
+      p = lane - slot * G;
+      Ln = (wi - pe * WPE) * LPW + slot;
+      lv = slot < LPW && p < NP && Ln < NPT && (int)blockIdx.x * EPB + pe < P.nElems;
+      lbase = slot * G;
+      if (!lv) { p = 0; Ln = 0; }
+    }
+    const int la = Ln % NP, lb = Ln / NP;
+    double* prec = sRow + NP + (size_t)pe * (RS + NACC) * NS;
+    double* pacc = prec + (size_t)RS * NS;
+#pragma unroll 1
+    for (int dir = 0; dir < 3; ++dir) {
+      const int stride = dir == 0 ? 1 : (dir == 1 ? NP : NPT);
+      const int base = dir == 0 ? NP * (la + NP * lb) : (dir == 1 ? la + NPT * lb : la + NP * lb);
+      const int own = base + p * stride, os = mpad<NP>(own);
+      double ro[NF], mo[3], racc[NE];
+#pragma unroll
+      for (int v = 0; v < NE; ++v) racc[v] = 0.;
+      if (lv) {
+#pragma unroll
+        for (int z = 0; z < NF; ++z) ro[z] = prec[os * RS + z];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) mo[c] = prec[os * RS + NQ + 3 * dir + c];
+      }
+#pragma unroll
+      for (int d = 1; d <= NP / 2; ++d) {
+        const bool active = lv && (2 * d < NP || p < d);
+        int q = p + d;
+        if (q >= NP) q -= NP;
+        // the pair's flux, then its contributions to the non-conservative sums of p and of q; an
+        // inactive lane's are zeros, so no selects are needed below
+        double F[NV], np[2] = {0., 0.}, nq[2] = {0., 0.};
+#pragma unroll
+        for (int v = 0; v < NV; ++v) F[v] = 0.;
+        if (active) {
+          // the partner's record is read in place (the log-mean logarithms only when needed)
+          const double* rq = prec + mpad<NP>(base + q * stride) * RS;
+          const double* mq = rq + NQ + 3 * dir;
+          pair_flux_mhd<VF>(P, ch, ro, rq, prec + os * RS, rq, mo, mq, F);
+          const double c0 = 0.5 * (mo[0] + mq[0]), c1 = 0.5 * (mo[1] + mq[1]), c2 = 0.5 * (mo[2] + mq[2]);
+          np[0] = c0 * rq[IB] + c1 * rq[IB + 1] + c2 * rq[IB + 2];
+          nq[0] = c0 * ro[IB] + c1 * ro[IB + 1] + c2 * ro[IB + 2];
+          np[1] = rq[IPSI];
+          nq[1] = ro[IPSI];
+        }
+        const double dOwn = sDvs[p * NP + q], dPart = sDvs[q * NP + p];
+        int src = p - d;
+        if (src < 0) src += NP;
+#pragma unroll
+        for (int v = 0; v < NE; ++v) {
+          racc[v] = fma(dOwn, v < NV ? F[v < NV ? v : 0] : np[v < NV ? 0 : v - NV], racc[v]);
+          racc[v] += __shfl_sync(0xffffffffu, dPart * (v < NV ? F[v < NV ? v : 0] : nq[v < NV ? 0 : v - NV]),
+                                 (lbase + src) & 31);
+        }
+      }
+      if (lv) {
+        racc[NV] += (mo[0] * ro[IB] + mo[1] * ro[IB + 1] + mo[2] * ro[IB + 2]) * sRow[p];
+        racc[NV + 1] = 0.5 * (mo[0] * ro[IV] + mo[1] * ro[IV + 1] + mo[2] * ro[IV + 2]) *
+                       (ro[IPSI] * sRow[p] + racc[NV + 1]);
+#pragma unroll
+        for (int v = 0; v < NE; ++v) pacc[os * NACC + v] += racc[v];
+      }
+      __syncthreads();
+    }
+  }
+  if (!valid) return;
+  const double* ac = acc + mpad<NP>(t) * NACC;
+  double ut[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) ut[v] = ac[v];
+  vol_finish_node<NP>(P, ch, e, t, u, ut, ac[NV], ac[NV + 1]);
 }
 
 // ------------------------------------------------------------------------------------------------
