@@ -107,6 +107,8 @@ struct KParams {
   // element kernels: blocks resident at once on the device (0: no prefetch); block b prefetches the
   // tile of block b + pfTiles into L2
   int pfTiles;
+  // the launches of this right-hand side may start early (launch_k): geometry is at rest in this stream
+  int pdl;
   // Gauss nodes: face states of ProlongToFace_U [side][master|slave][pt][5], the surface integral with
   // the split-form correction [elem][5][node] (added by the volume kernel instead of the LGL surface
   // terms), SurfMetrics [elem][6][3][pt] (mesh_vars.f90:67-70); all null for LGL
@@ -120,6 +122,32 @@ struct KParams {
   unsigned long long* instDtBits;    // [instance] CALCTIMESTEP minimum (bits of a double)
   int* instErrKey;                   // [instance] elem*8+errType of the first bad element
 };
+
+// Programmatic dependent launch.  A kernel launched with launch_k(pdl = true) may start while its
+// predecessor in the stream still drains: its blocks take the SM slots the predecessor no longer fills and
+// load what no kernel of a right-hand side writes (operators, connectivity, metrics); pdl_wait returns
+// when the predecessor has completed and its writes are visible, so every access to anything else stands
+// behind it.  Every kernel that is launched so calls pdl_wait in all threads (a successor's wait then
+// covers all earlier kernels too); pdl_trigger lets the successor start early.  Without the launch
+// attribute both do nothing.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... K, class... A>
+inline cudaError_t launch_k(bool pdl, void (*k)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                            A... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute a;
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &a;
+  c.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&c, k, K(args)...);
+}
 
 __device__ __forceinline__ bool halted(const KParams& P) { return P.haltFlag && *P.haltFlag != 0; }
 

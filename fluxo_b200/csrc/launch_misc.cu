@@ -121,8 +121,7 @@ static cudaError_t face_t(int NP, int nSides, cudaStream_t s, const KParams& P) 
   // 8 resident blocks of 128 threads per SM (64 registers): the face pass is DRAM-latency bound, and
   // the extra warps in flight outweigh the spills of the heavier Riemann solvers (measured at N=7 with
   // the matrix-dissipation solver: 4.2 TB/s against 3.5 TB/s at the unbounded 114 registers)
-  face_flux_kernel<RS, VISC, 8><<<grid, spb * npts, 0, s>>>(P, NP);
-  return cudaGetLastError();
+  return launch_k(P.pdl, face_flux_kernel<RS, VISC, 8>, grid, spb * npts, 0, s, P, NP);
 }
 
 cudaError_t launch_face_flux(int RS, bool visc, int NP, int nSides, cudaStream_t s, const KParams& P) {
@@ -142,8 +141,7 @@ cudaError_t launch_face_flux(int RS, bool visc, int NP, int nSides, cudaStream_t
 cudaError_t launch_lift_flux(int NP, int nSides, cudaStream_t s, const KParams& P) {
   const size_t n = (size_t)nSides * NP * NP;
   const int grid = (int)((n + 255) / 256);
-  lift_flux_kernel<<<grid, 256, 0, s>>>(P, NP, P.lflux);
-  return cudaGetLastError();
+  return launch_k(P.pdl, lift_flux_kernel, grid, 256, 0, s, P, NP, P.lflux);
 }
 
 cudaError_t launch_gradient(int NP, int nElems, cudaStream_t s, const KParams& P) {
@@ -154,8 +152,7 @@ template <int NP, bool VISC>
 static cudaError_t dt_t(int nElems, cudaStream_t s, const KParams& P, unsigned long long* dtBits, int* errKey) {
   constexpr int NP3 = NP * NP * NP;
   constexpr int EPB = (256 / NP3) > 0 ? (256 / NP3) : 1;
-  timestep_kernel<NP, VISC><<<(nElems + EPB - 1) / EPB, EPB * NP3, 0, s>>>(P, dtBits, errKey);
-  return cudaGetLastError();
+  return launch_k(P.pdl, timestep_kernel<NP, VISC>, (nElems + EPB - 1) / EPB, EPB * NP3, 0, s, P, dtBits, errKey);
 }
 
 cudaError_t launch_timestep(int NP, bool visc, int nElems, cudaStream_t s, const KParams& P,

@@ -17,8 +17,7 @@ static cudaError_t lv_t(int nElems, cudaStream_t s, const KParams& P) {
   if (e != cudaSuccess) return e;
   KParams Q = P;
   Q.pfTiles = resident_blocks(k, EPB * NP * NP * NP, smem, resident);
-  k<<<(nElems + EPB - 1) / EPB, EPB * NP * NP * NP, smem, s>>>(Q);
-  return cudaGetLastError();
+  return launch_k(P.pdl, k, (nElems + EPB - 1) / EPB, EPB * NP * NP * NP, smem, s, Q);
 }
 
 // N+1 = 8: the operator contractions on the FP64 tensor cores (lifting_mma.cuh), one element per block
@@ -32,8 +31,7 @@ static cudaError_t lv_mma_t(int nElems, cudaStream_t s, const KParams& P) {
   if (e != cudaSuccess) return e;
   KParams Q = P;
   Q.pfTiles = resident_blocks(k, 512, smem, resident);
-  k<<<nElems, 512, smem, s>>>(Q);
-  return cudaGetLastError();
+  return launch_k(P.pdl, k, nElems, 512, smem, s, Q);
 }
 
 template <int NP, int LIFT, int LV>

@@ -189,7 +189,7 @@ __device__ __forceinline__ void lv_node_fluxes(const KParams& P, int e, int t, i
 
 template <int NP, int LIFT, int LV>
 __global__ void __launch_bounds__(lv_epb<NP>() * NP * NP * NP, lv_minb<NP, LIFT>()) lift_visc_kernel(KParams P) {
-  if (halted(P)) return;
+  pdl_trigger();
   constexpr int NP3 = NP * NP * NP, NPT = NP * NP, N = NP - 1, EPB = lv_epb<NP>(), R = lv_row<NP>();
   extern __shared__ double smem[];
   double* sD = smem;             // D(i,l) at [i*R+l]
@@ -217,15 +217,19 @@ __global__ void __launch_bounds__(lv_epb<NP>() * NP * NP * NP, lv_minb<NP, LIFT>
       prefetch_l2_bulk(P.sJ + en * NP3, ne * sizeof(double));
     }
   }
-  double u[5];
   if (valid) {
     for (int z = t; z < 12; z += NP3) sE2S[eb][z] = P.e2s[12 * (size_t)e + z];  // NP3 = 8 for N = 1
-    const double* Ug = P.U + 5 * ((size_t)e * NP3 + t);
-#pragma unroll
-    for (int v = 0; v < 5; ++v) u[v] = Ug[v];
 #pragma unroll
     for (int c = 0; c < 9; ++c) prefetch_l2(P.metrics + (size_t)e * 9 * NP3 + c * NP3 + t);
     prefetch_l2(P.sJ + (size_t)e * NP3 + t);
+  }
+  pdl_wait();  // operators, connectivity and metrics above; from here on what earlier kernels wrote
+  if (halted(P)) return;
+  double u[5];
+  if (valid) {
+    const double* Ug = P.U + 5 * ((size_t)e * NP3 + t);
+#pragma unroll
+    for (int v = 0; v < 5; ++v) u[v] = Ug[v];
     double V[5];
     lifting_var_t<LV>(P, u, V);
 #pragma unroll

@@ -59,7 +59,7 @@ __device__ __forceinline__ void lm_tile(const double* a, const double* src, doub
 
 template <int LIFT, int LV>
 __global__ void __launch_bounds__(512, lv_minb<8, LIFT>()) lift_visc_mma_kernel(KParams P) {
-  if (halted(P)) return;
+  pdl_trigger();
   constexpr int NP = 8, NP3 = 512, NPT = 64, S = kLmStride;
   extern __shared__ double smem[];
   double* sV = smem;        // [5][S] lifting variable; later the divergence R[4][S]
@@ -83,12 +83,16 @@ __global__ void __launch_bounds__(512, lv_minb<8, LIFT>()) lift_visc_mma_kernel(
   const double* Ug = P.U + 5 * ((size_t)e * NP3 + t);
   if (valid) {
     if (t < 12) sE2S[t] = P.e2s[12 * (size_t)e + t];
-    double u[5];
-#pragma unroll
-    for (int v = 0; v < 5; ++v) u[v] = Ug[v];
 #pragma unroll
     for (int c = 0; c < 9; ++c) prefetch_l2(P.metrics + (size_t)e * 9 * NP3 + c * NP3 + t);
     prefetch_l2(P.sJ + (size_t)e * NP3 + t);
+  }
+  pdl_wait();  // connectivity and metrics above; from here on what earlier kernels wrote
+  if (halted(P)) return;
+  if (valid) {
+    double u[5];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) u[v] = Ug[v];
     double V[5];
     lifting_var_t<LV>(P, u, V);
 #pragma unroll

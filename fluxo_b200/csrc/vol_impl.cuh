@@ -22,8 +22,7 @@ static cudaError_t vol_shape_launch(int nElems, cudaStream_t s, const KParams& P
     const int grid = (nElems + EPB - 1) / EPB;
     KParams Q = P;
     Q.pfTiles = resident_blocks(k, threads, smem, resident);
-    k<<<grid, threads, smem, s>>>(Q);
-    return cudaGetLastError();
+    return launch_k(P.pdl, k, grid, threads, smem, s, Q);
   };
   if constexpr ((NP == 4 || NP == 6 || NP == 8) && LPW == 64 / NP)  // two nodes per thread
     return launch(volume_blk_kernel<NP, VF_ID, VISC, EPB, MINB>, VolBlkShape<NP, EPB>::THREADS,
