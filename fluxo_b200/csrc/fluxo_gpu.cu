@@ -290,7 +290,7 @@ void build_basis_tables(int N, BasisTables& B) {
 // Largest Euler / Navier-Stokes solve (nodes) whose launches start early (launch_k).  Its kernels are a few
 // waves each, so the gaps and prologues between them count: Euler N = 3 8^3 elements, 20 steps 2151 -> 2003 us,
 // Navier-Stokes N = 4 12^3 2112 -> 1949 us, N = 5 463 k nodes 203.5 -> 196.5 us.  Above, the early blocks only
-// take cache and shared memory from the running kernel: N = 7 32^3 step 22.8 -> 23.2 ms.
+// take cache and shared memory from the running kernel: N = 7 32^3 step 22.7 -> 23.2 ms.
 constexpr size_t kPdlNodes = (size_t)1 << 20;
 
 KParams base_params(fluxo_handle* h) {

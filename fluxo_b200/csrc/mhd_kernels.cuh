@@ -278,7 +278,7 @@ __device__ __forceinline__ void pair_flux_mhd(const KParams& P, double ch, const
 // with the pairs of the line, accumulated over the directions into one scalar each per node.  (The
 // diagonal of Dvs is zero.)  A separate pass over the line for them (8 shared loads per node of the line
 // and 13 multiply-adds) made the resistive N = 4 step on 24^3 elements 7.93 ms; riding along (two more
-// shuffled values per pair) 7.72 ms.
+// shuffled values per pair) 7.72 ms; the ideal N = 5 right-hand side (14x13x12) went from 181 to 171 us.
 // ------------------------------------------------------------------------------------------------
 template <int NP>
 __host__ __device__ constexpr int epb() { return (256 / (NP * NP * NP)) > 0 ? (256 / (NP * NP * NP)) : 1; }
