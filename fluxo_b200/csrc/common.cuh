@@ -133,6 +133,8 @@ struct KParams {
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// A refused launch is reported here and nowhere else: the thread's last error is cleared, so that a later
+// plain launch's cudaGetLastError() does not report it again.
 template <class... K, class... A>
 inline cudaError_t launch_k(bool pdl, void (*k)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
                             A... args) {
@@ -146,7 +148,9 @@ inline cudaError_t launch_k(bool pdl, void (*k)(K...), unsigned grid, unsigned b
   a.val.programmaticStreamSerializationAllowed = 1;
   c.attrs = &a;
   c.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&c, k, K(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&c, k, K(args)...);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
 }
 
 __device__ __forceinline__ bool halted(const KParams& P) { return P.haltFlag && *P.haltFlag != 0; }
