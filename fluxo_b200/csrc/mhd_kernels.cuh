@@ -279,6 +279,8 @@ __device__ __forceinline__ void pair_flux_mhd(const KParams& P, double ch, const
 // diagonal of Dvs is zero.)  A separate pass over the line for them (8 shared loads per node of the line
 // and 13 multiply-adds) made the resistive N = 4 step on 24^3 elements 7.93 ms; riding along (two more
 // shuffled values per pair) 7.72 ms; the ideal N = 5 right-hand side (14x13x12) went from 181 to 171 us.
+// NC = false (noncons = 0) is an instantiation without them; formed and thrown away they cost 4 to 6 % of a
+// step (ideal N = 7, 8^3 elements: 643 us per step with them, 604 us without).
 // ------------------------------------------------------------------------------------------------
 template <int NP>
 __host__ __device__ constexpr int epb() { return (256 / (NP * NP * NP)) > 0 ? (256 / (NP * NP * NP)) : 1; }
@@ -312,12 +314,12 @@ template <int NP>
 __host__ __device__ constexpr int vol_minb() { return vol_threads<NP>() <= 320 ? 2 : 1; }
 
 // Node epilogue of the volume kernel: from the line sums ut (split form), ncMHD and ncGLM
-// (non-conservative) of node t of element e to Ut (stage 0) or the LSERK update
-template <int NP>
+// (non-conservative; unused with HASNC = false) of node t of element e to Ut (stage 0) or the LSERK update
+template <int NP, bool HASNC>
 __device__ __forceinline__ void vol_finish_node(const KParams& P, double ch, int e, int t, const double* u, double* ut,
                                                 double ncMHD, double ncGLM) {
   constexpr int NP3 = NP * NP * NP, N = NP - 1, NPT = NP * NP;
-  const int NC = P.noncons;
+  const int NC = HASNC ? P.noncons : 0;
   const bool NCGLM = NC != 0 && P.ncGLM != 0;
   const int i = t % NP, j = (t / NP) % NP, k = t / NPT;
   if (NC != 0) {  // Phi(i) * sum of the line terms (Powell / Brackbill / Janhunen)
@@ -397,11 +399,12 @@ __device__ __forceinline__ void vol_finish_node(const KParams& P, double ch, int
   }
 }
 
-template <int NP, int VF>
+template <int NP, int VF, bool NC>
 __global__ void __launch_bounds__(vol_threads<NP>(), vol_minb<NP>()) volume_kernel(KParams P) {
   if (halted(P)) return;
   constexpr int NP3 = NP * NP * NP, NPT = NP * NP, EPB = epb<NP>(), LPW = vol_lpw<NP>();
-  constexpr int RS = Rec<VF>::RS, NQ = Rec<VF>::NQ, NF = Rec<VF>::NF, IB = Rec<VF>::B, IPSI = Rec<VF>::PSI, IV = Rec<VF>::V, NE = NV + 2;
+  constexpr int RS = Rec<VF>::RS, NQ = Rec<VF>::NQ, NF = Rec<VF>::NF, IB = Rec<VF>::B, IPSI = Rec<VF>::PSI, IV = Rec<VF>::V;
+  constexpr int NE = NC ? NV + 2 : NV;  // sums per line: Ut, then the non-conservative ones
   constexpr int NS = mpad_slots<NP>();
   extern __shared__ double smem[];
   double* sDvs = smem;        // Dvolsurf(i,l) at [i*NP+l]
@@ -485,11 +488,13 @@ __global__ void __launch_bounds__(vol_threads<NP>(), vol_minb<NP>()) volume_kern
           const double* rq = prec + mpad<NP>(base + q * stride) * RS;
           const double* mq = rq + NQ + 3 * dir;
           pair_flux_mhd<VF>(P, ch, ro, rq, prec + os * RS, rq, mo, mq, F);
-          const double c0 = 0.5 * (mo[0] + mq[0]), c1 = 0.5 * (mo[1] + mq[1]), c2 = 0.5 * (mo[2] + mq[2]);
-          np[0] = c0 * rq[IB] + c1 * rq[IB + 1] + c2 * rq[IB + 2];
-          nq[0] = c0 * ro[IB] + c1 * ro[IB + 1] + c2 * ro[IB + 2];
-          np[1] = rq[IPSI];
-          nq[1] = ro[IPSI];
+          if constexpr (NC) {
+            const double c0 = 0.5 * (mo[0] + mq[0]), c1 = 0.5 * (mo[1] + mq[1]), c2 = 0.5 * (mo[2] + mq[2]);
+            np[0] = c0 * rq[IB] + c1 * rq[IB + 1] + c2 * rq[IB + 2];
+            nq[0] = c0 * ro[IB] + c1 * ro[IB + 1] + c2 * ro[IB + 2];
+            np[1] = rq[IPSI];
+            nq[1] = ro[IPSI];
+          }
         }
         const double dOwn = sDvs[p * NP + q], dPart = sDvs[q * NP + p];
         int src = p - d;
@@ -502,9 +507,11 @@ __global__ void __launch_bounds__(vol_threads<NP>(), vol_minb<NP>()) volume_kern
         }
       }
       if (lv) {
-        racc[NV] += (mo[0] * ro[IB] + mo[1] * ro[IB + 1] + mo[2] * ro[IB + 2]) * sRow[p];
-        racc[NV + 1] = 0.5 * (mo[0] * ro[IV] + mo[1] * ro[IV + 1] + mo[2] * ro[IV + 2]) *
-                       (ro[IPSI] * sRow[p] + racc[NV + 1]);
+        if constexpr (NC) {
+          racc[NV] += (mo[0] * ro[IB] + mo[1] * ro[IB + 1] + mo[2] * ro[IB + 2]) * sRow[p];
+          racc[NV + 1] = 0.5 * (mo[0] * ro[IV] + mo[1] * ro[IV + 1] + mo[2] * ro[IV + 2]) *
+                         (ro[IPSI] * sRow[p] + racc[NV + 1]);
+        }
 #pragma unroll
         for (int v = 0; v < NE; ++v) pacc[os * NACC + v] += racc[v];
       }
@@ -516,7 +523,7 @@ __global__ void __launch_bounds__(vol_threads<NP>(), vol_minb<NP>()) volume_kern
   double ut[NV];
 #pragma unroll
   for (int v = 0; v < NV; ++v) ut[v] = ac[v];
-  vol_finish_node<NP>(P, ch, e, t, u, ut, ac[NV], ac[NV + 1]);
+  vol_finish_node<NP, NC>(P, ch, e, t, u, ut, ac[NV], ac[NV + 1]);
 }
 
 // ------------------------------------------------------------------------------------------------
