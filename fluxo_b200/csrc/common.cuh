@@ -107,7 +107,7 @@ struct KParams {
   // element kernels: blocks resident at once on the device (0: no prefetch); block b prefetches the
   // tile of block b + pfTiles into L2
   int pfTiles;
-  // the launches of this right-hand side may start early (launch_k): geometry is at rest in this stream
+  // how early the launches of this right-hand side may start (launch_k): geometry is at rest in this stream
   int pdl;
   // Gauss nodes: face states of ProlongToFace_U [side][master|slave][pt][5], the surface integral with
   // the split-form correction [elem][5][node] (added by the volume kernel instead of the LGL surface
@@ -123,20 +123,28 @@ struct KParams {
   int* instErrKey;                   // [instance] elem*8+errType of the first bad element
 };
 
-// Programmatic dependent launch.  A kernel launched with launch_k(pdl = true) may start while its
-// predecessor in the stream still drains: its blocks take the SM slots the predecessor no longer fills and
-// load what no kernel of a right-hand side writes (operators, connectivity, metrics); pdl_wait returns
-// when the predecessor has completed and its writes are visible, so every access to anything else stands
-// behind it.  Every kernel that is launched so calls pdl_wait in all threads (a successor's wait then
-// covers all earlier kernels too); pdl_trigger lets the successor start early.  Without the launch
-// attribute both do nothing.
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Programmatic dependent launch.  A kernel launched with launch_k(pdl != PDL_OFF) may start before its
+// predecessor in the stream has completed, and load what no kernel of a right-hand side writes (operators,
+// connectivity, metrics); pdl_wait returns when the predecessor has completed and its writes are visible, so
+// every access to anything else stands behind it.  Every kernel that is launched so calls pdl_wait in all
+// threads (a successor's wait then covers all earlier kernels too).  The successor's blocks come up
+//   PDL_TAIL   when the blocks of this kernel have ended: its launch overlaps the completion;
+//   PDL_DRAIN  when the last block of this kernel has started (pdl_trigger): its blocks take the SM slots
+//              that a last wave of this kernel leaves.
+// A kernel of less than a wave or two must not use PDL_DRAIN: its successor's blocks are placed beside all of
+// its own, so they share some SMs while others are idle, and the solve gets slower than without early
+// launches (fluxo_gpu.cu, pdl_mode; a launch shape that allows one block per SM only does not suffer).
+// Without the launch attribute pdl_trigger and pdl_wait do nothing.
+enum { PDL_OFF = 0, PDL_TAIL = 1, PDL_DRAIN = 2 };
+__device__ __forceinline__ void pdl_trigger(int pdl) {
+  if (pdl == PDL_DRAIN) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // A refused launch is reported here and nowhere else: the thread's last error is cleared, so that a later
 // plain launch's cudaGetLastError() does not report it again.
 template <class... K, class... A>
-inline cudaError_t launch_k(bool pdl, void (*k)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+inline cudaError_t launch_k(int pdl, void (*k)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
                             A... args) {
   cudaLaunchConfig_t c = {};
   c.gridDim = dim3(grid);
@@ -147,7 +155,7 @@ inline cudaError_t launch_k(bool pdl, void (*k)(K...), unsigned grid, unsigned b
   a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   a.val.programmaticStreamSerializationAllowed = 1;
   c.attrs = &a;
-  c.numAttrs = pdl ? 1 : 0;
+  c.numAttrs = pdl != PDL_OFF ? 1 : 0;
   const cudaError_t e = cudaLaunchKernelEx(&c, k, K(args)...);
   if (e != cudaSuccess) cudaGetLastError();
   return e;

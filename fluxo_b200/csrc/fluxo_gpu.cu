@@ -52,8 +52,8 @@ __global__ void td_begin_kernel(TDState* s, double t, double tEnd, int maxIter) 
 }
 
 // after CALCTIMESTEP: error check and dt clipping to tEnd (timedisc.f90:289-317)
-__global__ void td_finalize_kernel(TDState* s) {
-  pdl_trigger();
+__global__ void td_finalize_kernel(TDState* s, int pdl) {
+  pdl_trigger(pdl);
   pdl_wait();
   if (s->halt) return;
   if (s->errKey != INT_MAX) { s->err = s->errKey & 7; s->halt = 1; return; }
@@ -65,8 +65,8 @@ __global__ void td_finalize_kernel(TDState* s) {
 }
 
 // after the stages: t += dt, iteration count, termination (timedisc.f90:329-359)
-__global__ void td_advance_kernel(TDState* s) {
-  pdl_trigger();
+__global__ void td_advance_kernel(TDState* s, int pdl) {
+  pdl_trigger(pdl);
   pdl_wait();
   if (s->halt) return;
   if (s->errKey != INT_MAX) { s->err = s->errKey & 7; s->halt = 1; return; }  // NFVSE_CORR during the step
@@ -287,18 +287,22 @@ void build_basis_tables(int N, BasisTables& B) {
   for (int i = 0; i < NP; ++i) { B.wGP[i] = b.w[i]; B.xGP[i] = b.x[i]; }
 }
 
-// Largest Euler / Navier-Stokes solve (nodes) whose launches start early (launch_k).  Its kernels are a few
-// waves each, so the gaps and prologues between them count: Euler N = 3 8^3 elements, 20 steps 2151 -> 2003 us,
-// Navier-Stokes N = 4 12^3 2112 -> 1949 us, N = 5 463 k nodes 203.5 -> 196.5 us.  Above, the early blocks only
-// take cache and shared memory from the running kernel: N = 7 32^3 step 22.7 -> 23.2 ms.
-constexpr size_t kPdlNodes = (size_t)1 << 20;
+// How early the launches of an Euler / Navier-Stokes solve of `nodes` own nodes start (PDL_*, common.cuh).
+// us per step without / PDL_TAIL / PDL_DRAIN, at the best launch shape of each:
+//   up to 2^18 nodes the kernels are a wave or two: N = 3 Euler 8^3 elements 117 / 88 / 107, N = 7
+//   Navier-Stokes 5^3 260 / 215 / 290 (N = 1 16^3: 193 / 146 / 224), N = 5 8^3 319 / 271 / 301;
+//   up to 2^20 their drain is worth filling: N = 3 Euler 20^3 492 / 473 / 461, N = 7 10^3 533 / 512 / 489;
+//   above, the early blocks only take cache and shared memory from the running kernel: N = 7 32^3 22.7 ms
+//   without, 23.2 ms with PDL_DRAIN.
+constexpr size_t kPdlDrainNodes = (size_t)1 << 18, kPdlNodes = (size_t)1 << 20;
+int pdl_mode(size_t nodes) { return nodes > kPdlNodes ? PDL_OFF : (nodes >= kPdlDrainNodes ? PDL_DRAIN : PDL_TAIL); }
 
 KParams base_params(fluxo_handle* h) {
   KParams P{};
   const fluxo_cfg& c = h->cfg;
   P.nElems = h->nOwn; P.nSides = h->nSides;
   P.U = h->dU; P.Ut = h->dUt; P.UtTmp = h->dUtTmp; P.grad = nullptr; P.utvisc = h->dUtVisc;
-  P.pdl = !h->mhd && (size_t)h->nOwn * h->NP * h->NP * h->NP <= kPdlNodes;
+  P.pdl = h->mhd ? PDL_OFF : pdl_mode((size_t)h->nOwn * h->NP * h->NP * h->NP);
   P.metrics = h->dMetrics; P.sJ = h->dsJ; P.facegeo = h->dFaceGeo; P.xGP = h->dXGP;
   P.s2e = h->dS2E; P.e2s = h->dE2S;
   P.flux = h->dFlux; P.lflux = h->dLFlux; P.gtrace = h->dGTrace;
@@ -977,9 +981,9 @@ int fluxo_gpu_time_disc(fluxo_handle* h, double t, double tEnd, int maxIter, dou
         else FLUXO_CUDA(h, launch_timestep(h->NP, h->visc, h->nOwn, s, P, &td->dtBits, &td->errKey));
       }
       if ((r = exchange(h, FLUXO_XCHG_DT, &td->dtBits, &td->errKey))) return r;
-      FLUXO_CUDA(h, launch_k(P.pdl, td_finalize_kernel, 1, 1, 0, s, td));
+      FLUXO_CUDA(h, launch_k(P.pdl, td_finalize_kernel, 1, 1, 0, s, td, P.pdl));
       if ((r = rk_step(h, 0., 0., &td->dt, &td->halt, h->mhd ? &td->ch : nullptr, &td->errKey))) return r;
-      FLUXO_CUDA(h, launch_k(P.pdl, td_advance_kernel, 1, 1, 0, s, td));
+      FLUXO_CUDA(h, launch_k(P.pdl, td_advance_kernel, 1, 1, 0, s, td, P.pdl));
       h->launches += 3;
       if (maxIter > 0 && ++enqueued >= maxIter) break;
     }

@@ -30,7 +30,7 @@ __device__ __forceinline__ int boundary_sides(int i, int j, int k, int N, int* s
 // ------------------------------------------------------------------------------------------------
 template <int RS, bool VISC>
 __device__ __forceinline__ void face_flux_body(const KParams& P, int NP) {
-  pdl_trigger();
+  pdl_trigger(P.pdl);
   pdl_wait();
   if (halted(P)) return;
   const int npts = NP * NP;
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(128, MINB) face_flux_kernel(KParams P, int NP)
 // lflux = 1/2 (V_slave - V_master) * SurfElem; the normal components are applied where consumed.
 // ------------------------------------------------------------------------------------------------
 static __global__ void lift_flux_kernel(KParams P, int NP, double* lf) {
-  pdl_trigger();
+  pdl_trigger(P.pdl);
   pdl_wait();
   if (halted(P)) return;
   const int npts = NP * NP;
@@ -286,7 +286,7 @@ __device__ __forceinline__ void vol_finish_node(const KParams& P, int e, int t, 
 template <int NP, int VF, bool VISC, int EPB, int LPW, int MINB, int OWNSM>
 __global__ void __launch_bounds__(VolShape<NP, EPB, LPW>::THREADS, VolShape<NP, EPB, LPW, MINB>::MINB)
 volume_kernel(KParams P) {
-  pdl_trigger();
+  pdl_trigger(P.pdl);
   pdl_wait();
   if (halted(P)) return;
   constexpr int NP3 = NP * NP * NP, NPT = NP * NP;
@@ -482,7 +482,7 @@ __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
 
 template <int NP, int VF, bool VISC, int EPB, int MINB>
 __global__ void __launch_bounds__(VolBlkShape<NP, EPB>::THREADS, MINB) volume_blk_kernel(KParams P) {
-  pdl_trigger();
+  pdl_trigger(P.pdl);
   using SH = VolBlkShape<NP, EPB>;
   constexpr int NP3 = NP * NP * NP, NPT = NP * NP, G = SH::G, LPW = SH::LPW, NS = vb_slots<NP>();
   constexpr int RS = VolRec<VF>::RS, NF = VolRec<VF>::NF, MO = VolRec<VF>::MO, NODES = EPB * NP3;
@@ -673,7 +673,7 @@ __global__ void __launch_bounds__(VolBlkShape<NP, EPB>::THREADS, MINB) volume_bl
 // ------------------------------------------------------------------------------------------------
 template <int NP, bool VISC>
 __global__ void __launch_bounds__(512) timestep_kernel(KParams P, unsigned long long* dtBits, int* errKey) {
-  pdl_trigger();
+  pdl_trigger(P.pdl);
   pdl_wait();
   if (halted(P)) return;
   constexpr int NP3 = NP * NP * NP;

@@ -189,7 +189,7 @@ __device__ __forceinline__ void lv_node_fluxes(const KParams& P, int e, int t, i
 
 template <int NP, int LIFT, int LV>
 __global__ void __launch_bounds__(lv_epb<NP>() * NP * NP * NP, lv_minb<NP, LIFT>()) lift_visc_kernel(KParams P) {
-  pdl_trigger();
+  pdl_trigger(P.pdl);
   constexpr int NP3 = NP * NP * NP, NPT = NP * NP, N = NP - 1, EPB = lv_epb<NP>(), R = lv_row<NP>();
   extern __shared__ double smem[];
   double* sD = smem;             // D(i,l) at [i*R+l]

@@ -59,7 +59,7 @@ __device__ __forceinline__ void lm_tile(const double* a, const double* src, doub
 
 template <int LIFT, int LV>
 __global__ void __launch_bounds__(512, lv_minb<8, LIFT>()) lift_visc_mma_kernel(KParams P) {
-  pdl_trigger();
+  pdl_trigger(P.pdl);
   constexpr int NP = 8, NP3 = 512, NPT = 64, S = kLmStride;
   extern __shared__ double smem[];
   double* sV = smem;        // [5][S] lifting variable; later the divergence R[4][S]
