@@ -514,7 +514,7 @@ def kernel_rooflines(kinds, N, nd, nElems, fp64_peak):
 
 
 def shape_dict(N, volume_flux, visc):
-    """The volume kernel's launch shape the autotuner chose (index -1: not tuned)."""
+    """The volume kernel's launch shape of the last launch (index -1: none)."""
     from fluxo_b200.solver import volume_shape
 
     count, index, epb, lpw = volume_shape(N, volume_flux, visc)
@@ -815,7 +815,7 @@ def run_tgv_trace(args):
     nd = op.nElems * (w["N"] + 1) ** 3
     _, _, stream_ptr = op.device_buffers()
     stream = torch.cuda.ExternalStream(stream_ptr, device=dev)
-    op.dg_time_derivative(0.0)  # first use: the volume kernel's launch-shape tuning happens here
+    op.dg_time_derivative(0.0)
     barrier(world)
     torch.cuda.synchronize(dev)
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)

@@ -30,6 +30,7 @@
 #include "host_setup.h"
 #include "host_copy.h"
 #include "launch.h"
+#include "vol_shapes.h"
 
 using namespace fluxo;
 
@@ -126,6 +127,7 @@ struct Group {
   fluxo_cfg key{};
   int N = 0, NP = 0;
   bool visc = false;
+  int volShape = 0;  // launch shape of the volume kernel that each member also runs alone (vol_shapes.h)
   int nStages = 0;
   double RKA[24]{}, RKb[24]{}, RKc[24]{}, CFLScale = 0., DFLScale = 0.;
   int nElems = 0, nSides = 0;
@@ -260,7 +262,7 @@ cudaError_t enqueue_group_step(const fluxo_batch* b, const Group& g, cudaStream_
       if ((e = launch_gradient(g.NP, g.nElems, s, P)) != cudaSuccess) return e;
     }
     if ((e = launch_face_flux(g.key.riemann, g.visc, g.NP, g.nSides, s, P)) != cudaSuccess) return e;
-    if ((e = launch_volume(g.NP, g.key.volume_flux, g.visc, g.nElems, s, P)) != cudaSuccess) return e;
+    if ((e = launch_volume(g.NP, g.key.volume_flux, g.visc, g.volShape, g.nElems, s, P)) != cudaSuccess) return e;
   }
   batch_advance_kernel<<<nb, bs, 0, s>>>(g.slot0, n, b->dState);
   return cudaGetLastError();
@@ -315,12 +317,14 @@ int commit(fluxo_batch* b) {
     Instance& I = kv.second;
     if (I.placed || I.removed) continue;
     const fluxo_cfg key = group_key(I.cfg);
+    const bool visc = I.cfg.eqn == FLUXO_EQN_NAVIERSTOKES;
+    const int shape = vol_shape_rule(I.cfg.N + 1, I.cfg.volume_flux, visc, I.nElems);
     int gi = -1;
     for (size_t k = 0; k < ng.size(); ++k)
-      if (std::memcmp(&ng[k].key, &key, sizeof(key)) == 0) gi = (int)k;
+      if (ng[k].volShape == shape && std::memcmp(&ng[k].key, &key, sizeof(key)) == 0) gi = (int)k;
     if (gi < 0) {
       Group g;
-      g.key = key; g.N = I.cfg.N; g.NP = I.cfg.N + 1; g.visc = (I.cfg.eqn == FLUXO_EQN_NAVIERSTOKES);
+      g.key = key; g.N = I.cfg.N; g.NP = I.cfg.N + 1; g.visc = visc; g.volShape = shape;
       time_disc_setup(I.cfg, g.RKA, g.RKb, g.RKc, &g.nStages, &g.CFLScale, &g.DFLScale);
       BasisTables hb;
       basis_tables_for(g.N, hb);
@@ -458,10 +462,6 @@ int commit(fluxo_batch* b) {
     BATCH_CUDA(b, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     b->joins.push_back(ev);
   }
-  // launch shapes of the volume kernels, tuned on the group's own arrays before the capture
-  for (const Group& g : b->groups)
-    if (g.nElems > 0 && volume_shape(g.NP, g.key.volume_flux, g.visc) < 0)
-      BATCH_CUDA(b, tune_volume(g.NP, g.key.volume_flux, g.visc, g.nElems, s, group_params(b, g)));
   // the step graph itself is captured by the first fluxo_batch_run after this (a server that only
   // runs device-resident loops captures the loop graph alone)
   b->dirty = false;

@@ -488,13 +488,10 @@ int rhs(fluxo_handle* h, KParams P) {
     FLUXO_CUDA(h, launch_gauss_surf(h->NP, h->cfg.volume_flux, h->nOwn, s, P));
     h->launches += 1;
   }
-  if (volume_shape(h->NP, h->cfg.volume_flux, h->visc) < 0) {  // first RHS of this (N, flux, visc)
-    FLUXO_CUDA(h, tune_volume(h->NP, h->cfg.volume_flux, h->visc, h->nOwn, s, P));
-    if (volume_shape_count(h->NP) > 1) h->launches += 4 * volume_shape_count(h->NP);
-  }
   {
     ProfScope ps(h, 3);
-    FLUXO_CUDA(h, launch_volume(h->NP, h->cfg.volume_flux, h->visc, h->nOwn, s, P));
+    const int vf = h->cfg.volume_flux;
+    FLUXO_CUDA(h, launch_volume(h->NP, vf, h->visc, vol_shape_rule(h->NP, vf, h->visc, h->nOwn), h->nOwn, s, P));
   }
   h->launches += 2;
   return FLUXO_OK;

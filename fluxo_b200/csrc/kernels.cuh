@@ -150,17 +150,17 @@ static __global__ void lift_flux_kernel(KParams P, int NP, double* lf) {
 // adds its sum to its shared accumulator.
 //
 // The partner's share of each pair flux travels by warp shuffle to the partner's lane, so a line must
-// live in one warp.  Launch shape (template parameters, chosen per N by the launcher's autotuner):
+// live in one warp.  Launch shape (template parameters, chosen by vol_shape_rule, vol_shapes.h):
 // EPB elements per block and the line-to-warp schedule of the pair phase,
 //   LPW = 0: thread t of an element takes node t's line position in every direction (lines are
 //            contiguous in the thread index; needs NP | 32);
 //   LPW > 0: LPW lines per warp, line slot s on lanes [s*G, s*G+NP) with G = 32/LPW, the other lanes
 //            idle; the block then has more threads than nodes and the node phases use the first
 //            EPB*NP^3 threads.
-// Every schedule adds the same terms in the same order; the shapes are separate instantiations,
-// though, and the compiler may fuse a different product of an a*b + c*d into a multiply-add in each,
-// so shapes agree to roundoff (one process uses one shape per N, flux and viscosity, so batched and
-// single solves stay bit-identical).
+// Every schedule of this kernel adds the same terms in the same order; the shapes are separate
+// instantiations, though, and the compiler may fuse a different product of an a*b + c*d into a multiply-add
+// in each, so shapes agree to roundoff only.  The shape follows from the solve alone, in a batch too, so
+// batched and single solves stay bit-identical.
 // ------------------------------------------------------------------------------------------------
 template <int NP>
 __host__ __device__ constexpr int vol_epb() { return (256 / (NP * NP * NP)) > 0 ? (256 / (NP * NP * NP)) : 1; }

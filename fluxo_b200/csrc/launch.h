@@ -14,10 +14,10 @@ struct LaunchError {
   cudaError_t err;
 };
 
-// Volume kernel: NP in 2..9, VF in {0,1,2,5,10,32}, in the launch shape the autotuner chose for
-// (NP, VF, visc) (vol_shapes.h; shape 0 until tuned or pinned).  Returns cudaErrorInvalidValue for
-// unsupported combinations.
-cudaError_t launch_volume(int NP, int VF, bool visc, int nElems, cudaStream_t s, const KParams& P);
+// Volume kernel: NP in 2..9, every volume flux of volume_flux_supported, over nElems elements of solves
+// that run launch shape `rule` (vol_shape_rule of vol_shapes.h), or in the shape pinned for (NP, VF, visc).
+// Returns cudaErrorInvalidValue for unsupported combinations.
+cudaError_t launch_volume(int NP, int VF, bool visc, int rule, int nElems, cudaStream_t s, const KParams& P);
 cudaError_t launch_volume_shape(int NP, int VF, bool visc, int shape, int nElems, cudaStream_t s,
                                 const KParams& P);
 cudaError_t launch_volume_vf0(int NP, bool visc, int shape, int nElems, cudaStream_t s, const KParams& P);
@@ -32,12 +32,7 @@ cudaError_t launch_volume_vf8(int NP, bool visc, int shape, int nElems, cudaStre
 cudaError_t launch_volume_vf9(int NP, bool visc, int shape, int nElems, cudaStream_t s, const KParams& P);
 cudaError_t launch_volume_vf10(int NP, bool visc, int shape, int nElems, cudaStream_t s, const KParams& P);
 cudaError_t launch_volume_vf32(int NP, bool visc, int shape, int nElems, cudaStream_t s, const KParams& P);
-// Autotuner of the volume kernel's launch shape: times every candidate shape of (NP, VF, visc) on the
-// given data (stage-0 launches, which write only Ut) and keeps the fastest for the process; a no-op
-// once (NP, VF, visc) is tuned or pinned, or when it has one candidate.  Not callable during stream
-// capture (it synchronises the stream).
-cudaError_t tune_volume(int NP, int VF, bool visc, int nElems, cudaStream_t s, const KParams& P);
-// Chosen shape (-1: not tuned), pin (shape < 0: back to untuned), candidate count.
+// Pinned shape, or that of the last launch (-1: none yet); pin (shape < 0: back to the rule); shape count.
 int volume_shape(int NP, int VF, bool visc);
 bool pin_volume_shape(int NP, int VF, bool visc, int shape);
 int volume_shape_count(int NP);

@@ -1,6 +1,6 @@
 // Launchers of the face, lifting and time-step kernels, the volume-flux dispatcher and the volume
-// kernel's launch-shape autotuner.
-#include <mutex>
+// kernel's launch shapes.
+#include <atomic>
 
 #include "kernels.cuh"
 #include "launch.h"
@@ -28,74 +28,33 @@ cudaError_t launch_volume_shape(int NP, int VF, bool visc, int shape, int nElems
 }
 
 namespace {
-// chosen launch shape per (NP, VF, visc); -1 = not tuned
-std::mutex g_shape_mutex;
-int g_shape[10][33][2];
-bool g_shape_init = false;
+// per (NP, VF, visc), shape + 1: the pinned one (0: none, the rule decides) and that of the last launch (for
+// reports only)
+std::atomic<int> g_pinned[10][33][2], g_used[10][33][2];
 
-int* shape_slot(int NP, int VF, bool visc) {
-  if (NP < 2 || NP > 9 || VF < 0 || VF > 32) return nullptr;
-  if (!g_shape_init) {
-    for (auto& a : g_shape)
-      for (auto& b : a) b[0] = b[1] = -1;
-    g_shape_init = true;
-  }
-  return &g_shape[NP][VF][visc ? 1 : 0];
-}
+bool shape_key(int NP, int VF) { return NP >= 2 && NP <= 9 && VF >= 0 && VF <= 32; }
 }  // namespace
 
 int volume_shape_count(int NP) { return vol_shape_count(NP); }
 
 int volume_shape(int NP, int VF, bool visc) {
-  std::lock_guard<std::mutex> lk(g_shape_mutex);
-  int* p = shape_slot(NP, VF, visc);
-  return p ? *p : -1;
+  if (!shape_key(NP, VF)) return -1;
+  const int pin = g_pinned[NP][VF][visc].load();
+  return (pin ? pin : g_used[NP][VF][visc].load()) - 1;
 }
 
 bool pin_volume_shape(int NP, int VF, bool visc, int shape) {
-  std::lock_guard<std::mutex> lk(g_shape_mutex);
-  int* p = shape_slot(NP, VF, visc);
-  if (!p || shape >= vol_shape_count(NP)) return false;
-  *p = shape < 0 ? -1 : shape;
+  if (!shape_key(NP, VF) || shape >= vol_shape_count(NP)) return false;
+  g_pinned[NP][VF][visc].store(shape < 0 ? 0 : shape + 1);
+  if (shape < 0) g_used[NP][VF][visc].store(0);
   return true;
 }
 
-cudaError_t launch_volume(int NP, int VF, bool visc, int nElems, cudaStream_t s, const KParams& P) {
-  const int sh = volume_shape(NP, VF, visc);
-  return launch_volume_shape(NP, VF, visc, sh < 0 ? 0 : sh, nElems, s, P);
-}
-
-cudaError_t tune_volume(int NP, int VF, bool visc, int nElems, cudaStream_t s, const KParams& P) {
-  const int C = vol_shape_count(NP);
-  if (volume_shape(NP, VF, visc) >= 0) return cudaSuccess;
-  if (C <= 1) {
-    pin_volume_shape(NP, VF, visc, 0);
-    return cudaSuccess;
-  }
-  KParams Q = P;
-  Q.stage = 0;           // writes Ut only: the state and the RK register stay untouched
-  Q.haltFlag = nullptr;  // every launch does its full work
-  Q.grad = nullptr;
-  cudaEvent_t a, b;
-  cudaError_t e;
-  if ((e = cudaEventCreate(&a)) != cudaSuccess) return e;
-  if ((e = cudaEventCreate(&b)) != cudaSuccess) { cudaEventDestroy(a); return e; }
-  int best = 0;
-  float bestMs = 0.f;
-  for (int i = 0; i < C && e == cudaSuccess; ++i) {
-    if ((e = launch_volume_shape(NP, VF, visc, i, nElems, s, Q)) != cudaSuccess) break;  // warm-up
-    if ((e = cudaEventRecord(a, s)) != cudaSuccess) break;
-    for (int r = 0; r < 3 && e == cudaSuccess; ++r) e = launch_volume_shape(NP, VF, visc, i, nElems, s, Q);
-    if (e != cudaSuccess) break;
-    if ((e = cudaEventRecord(b, s)) != cudaSuccess || (e = cudaEventSynchronize(b)) != cudaSuccess) break;
-    float ms = 0.f;
-    if ((e = cudaEventElapsedTime(&ms, a, b)) != cudaSuccess) break;
-    if (i == 0 || ms < bestMs) { bestMs = ms; best = i; }
-  }
-  cudaEventDestroy(a);
-  cudaEventDestroy(b);
-  if (e == cudaSuccess) pin_volume_shape(NP, VF, visc, best);
-  return e;
+cudaError_t launch_volume(int NP, int VF, bool visc, int rule, int nElems, cudaStream_t s, const KParams& P) {
+  if (!shape_key(NP, VF)) return cudaErrorInvalidValue;
+  const int pin = g_pinned[NP][VF][visc].load(), shape = pin ? pin - 1 : rule;
+  g_used[NP][VF][visc].store(shape + 1);
+  return launch_volume_shape(NP, VF, visc, shape, nElems, s, P);
 }
 
 bool volume_flux_supported(int VF) {

@@ -26,6 +26,7 @@
 #include "../../include/fluxo_gpu.h"
 #include "common.cuh"
 #include "launch.h"
+#include "vol_shapes.h"
 
 using namespace fluxo;
 
@@ -154,7 +155,8 @@ extern "C" int fluxo_gpu_dg_time_derivative_noalloc(const fluxo_cfg* cfg, int nE
   P.stage = 0;  // plain DGTimeDerivative: the volume kernel writes Ut
 
   if ((e = launch_face_flux(cfg->riemann, false, NP, nSides, s, P)) != cudaSuccess ||
-      (e = launch_volume(NP, cfg->volume_flux, false, nElems, s, P)) != cudaSuccess)
+      (e = launch_volume(NP, cfg->volume_flux, false, vol_shape_rule(NP, cfg->volume_flux, false, nElems), nElems, s, P)) !=
+          cudaSuccess)
     return bad(FLUXO_ECUDA, std::string("launch: ") + cudaGetErrorString(e));
   e = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = cudaGetLastError();

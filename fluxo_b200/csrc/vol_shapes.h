@@ -1,13 +1,13 @@
-// Candidate launch shapes of the Euler / Navier-Stokes volume kernel per N+1, for the autotuner:
+// Launch shapes of the Euler / Navier-Stokes volume kernel per N+1:
 //   epb   elements per block;
 //   lpw   lines per warp in the pair phase (0: lines contiguous in the thread index, needs N+1 | 32);
 //         64/(N+1) for N+1 = 4, 6, 8 selects the kernel with two nodes of a line per thread;
 //   minb  resident blocks per SM the register allocation must allow (0: 2 up to 512 threads, else 1);
 //   ownsm 1: a thread reads its own node's record from shared memory in every round instead of
 //         holding it in registers (fewer registers, more shared-memory loads).
-// Entry 0 of each list is the shape used before tuning.  All shapes of one N add the same terms (the
-// one-node ones also in the same order); they agree to roundoff and differ in occupancy, idle lanes,
-// register spills and shared-memory traffic.
+// All shapes of one N add the same terms, the one-node ones also in the same order; they agree to roundoff
+// and differ in occupancy, idle lanes, register spills and shared-memory traffic.  vol_shape_rule says which
+// one a solve runs.
 #pragma once
 
 namespace fluxo {
@@ -36,6 +36,30 @@ constexpr int vol_shape_count(int NP) {
   int c = 0;
   while (NP >= 0 && NP < 10 && c < kVolShapeMax && kVolShapes[NP][c].epb > 0) ++c;
   return c;
+}
+
+// The shape that a solve of nElems elements runs: a function of its configuration and size alone, so that its
+// results do not depend on what else the process ran, nor on a timing.  A batch keeps solves of different
+// shapes in different groups, so an instance runs the shape that it would run alone.
+//
+// One shape per N, but for N = 3.  us per step, best of repeated legs of the time loop, EC-KEP flux unless said:
+//   N = 1: {16} as fast or faster at every size (40^3 Euler 636, {32} 662);
+//   N = 2: {8,10} (27^3 Euler 605; {8,8} 717, {4,8} 730; at 4^3 84, 89, 83);
+//   N = 4: {2,6} (16^3 Navier-Stokes 1065; {2,4} 1083, {1,4} 1305; at 4^3 158, 163, 155);
+//   N = 5: two nodes per thread, {1,10,4} (14^3 Euler 579; {2,10,2} 581, one node 731; at 4^3 113, 113, 98);
+//   N = 6: {1,4} (13^3 Euler 779; {1,4,1} 1097, {1,4,0,1} 784; at 4^3 104, 102, 103);
+//   N = 7: two nodes per thread (12^3 Navier-Stokes 1371, one node 1482; at 4^3 217, 210).
+// The shape that is faster on a few elements is not used there where it is much slower on many: the tiny
+// solves of a batch share one launch.
+//   N = 3: one node per thread, {2}, up to a few waves (8^3 Euler 88, two nodes 104); two nodes, {1,16,16},
+//   above 2^20 nodes (40^3 Euler 2617, one node 2695; Kennedy-Gruber 2491, 2750; Navier-Stokes 5743, 5773),
+//   and from 2^18 for Euler (20^3 407, 414).  Between, where launches start while the last wave of their
+//   predecessor drains (pdl_mode), one node is faster for Navier-Stokes (20^3 858, 870) and for the longer
+//   records of standard DG, dealiased metrics and Ducros (20^3 Euler 420, 479).
+constexpr int vol_shape_rule(int NP, int VF, bool visc, int nElems) {
+  if (NP == 4)
+    return nElems > (1 << 14) || (nElems >= (1 << 12) && !visc && VF != 0 && VF != 1 && VF != 3) ? 1 : 2;
+  return NP == 2 ? 1 : 0;
 }
 
 }  // namespace fluxo

@@ -357,7 +357,7 @@ def fp64_peak(device=0):
 
 
 def volume_shape(N, volume_flux, visc=False):
-    """(candidate count, chosen index or -1, elements per block, lines per warp) of the volume kernel."""
+    """(shape count, index pinned or last launched or -1, elements per block, lines per warp) of the volume kernel."""
     c, i, e, l = (ctypes.c_int() for _ in range(4))
     _lib.check(_lib.load().fluxo_gpu_volume_shape(int(N), int(volume_flux), int(bool(visc)), ctypes.byref(c),
                                                   ctypes.byref(i), ctypes.byref(e), ctypes.byref(l)))
@@ -365,5 +365,5 @@ def volume_shape(N, volume_flux, visc=False):
 
 
 def set_volume_shape(N, volume_flux, visc, index):
-    """Pins the volume kernel's launch shape of (N, volume_flux, visc); index < 0 re-enables tuning."""
+    """Pins the volume kernel's launch shape of (N, volume_flux, visc); index < 0: back to the rule."""
     _lib.check(_lib.load().fluxo_gpu_set_volume_shape(int(N), int(volume_flux), int(bool(visc)), int(index)))

@@ -266,12 +266,13 @@ int fluxo_gpu_launch_count(fluxo_handle* h, uint64_t* n);
 int fluxo_gpu_set_profiling(fluxo_handle* h, int enable);
 int fluxo_gpu_get_profile(fluxo_handle* h, int kind, double* total_ms, uint64_t* count);
 
-/* Launch shape of the Euler / Navier-Stokes volume kernel (no counterpart in the reference): for each
- * (N, volume_flux, visc) a few candidate shapes (elements per block, lines per warp; 0 = lines
- * contiguous in the thread index) give identical results; the first right-hand side of a handle, or
- * the first run of a batch group, times them on its own data and keeps the fastest for the process.
- * fluxo_gpu_volume_shape reports the candidates, the chosen index (-1: not tuned yet) and its shape;
- * fluxo_gpu_set_volume_shape pins one (index < 0: tune again at the next use). */
+/* Launch shape of the Euler / Navier-Stokes volume kernel (no counterpart in the reference): for each N
+ * there are a few shapes (elements per block, lines per warp; 0 = lines contiguous in the thread index),
+ * whose results agree to roundoff (the order of a node's sums may differ).  A solve's shape follows from
+ * its N, volume_flux, visc and element count alone, also as an instance of a batch.
+ * fluxo_gpu_volume_shape reports the number of shapes, the index of the pinned one or else of the last
+ * launch of (N, volume_flux, visc) in this process (-1: none yet) and that shape;
+ * fluxo_gpu_set_volume_shape pins one for every size (index < 0: back to the rule). */
 int fluxo_gpu_volume_shape(int N, int volume_flux, int visc, int* count, int* index, int* epb, int* lpw);
 int fluxo_gpu_set_volume_shape(int N, int volume_flux, int visc, int index);
 

@@ -1,6 +1,7 @@
 """Launch shapes of the volume kernel (vol_shapes.h): every candidate of an N matches the oracle and
-the other candidates to roundoff (the shapes are separate instantiations whose multiply-add fusion
-may differ), the autotuner picks one of them, and a process keeps using it (same bits on re-use)."""
+the other candidates to roundoff (the shapes are separate instantiations whose multiply-add fusion may
+differ, and the two-node ones sum in another order), and without a pin a solve runs one of them (same bits on
+re-use)."""
 import numpy as np
 import pytest
 
@@ -37,11 +38,11 @@ def test_every_shape_same_bits(gpu_lib, N, eqn, vf):
     for o in outs:
         assert np.linalg.norm(o - ref) / np.linalg.norm(ref) <= 1e-12
         assert np.linalg.norm(o - outs[0]) / np.linalg.norm(outs[0]) <= 1e-14
-    set_volume_shape(N, vf, eqn == 1, -1)   # the next RHS tunes again
+    set_volume_shape(N, vf, eqn == 1, -1)   # back to the rule
     op.dg_time_derivative(0.0)
     cnt, chosen, epb, lpw = volume_shape(N, vf, eqn == 1)
     assert 0 <= chosen < cnt and epb >= 1
     assert np.array_equal(op.get_ut(), outs[chosen])
-    op.dg_time_derivative(0.0)             # the tuned shape stays: same bits
+    op.dg_time_derivative(0.0)             # the shape stays: same bits
     assert np.array_equal(op.get_ut(), outs[chosen])
     op.close()
