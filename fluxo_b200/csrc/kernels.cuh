@@ -181,7 +181,7 @@ __host__ __device__ constexpr int vol_slot(int n) { return n + (n >> 4); }
 // The Euler / Navier-Stokes kernel's node padding per (N+1, lines per warp): chosen with a lane-by-
 // lane model of the pair rounds (own and partner records and accumulators of all three directions)
 // so that a warp's 8-byte accesses need the minimum number of shared wavefronts (one spare slot
-// every 16 nodes needs 1.6-2x as many): N+1 = 8 contiguous, 4 contiguous, 5/6/7 with 4 lines per
+// every 16 nodes needs 1.6-2x as many): N+1 = 8 contiguous, 4 contiguous, 5 and 7 with 4 lines per
 // warp and 3 with 8 lines per warp are conflict-free (7: 1.04, 3: 1.08); the other schedules keep
 // the 16-node padding.
 template <int NP, int LPW = 0>
@@ -189,7 +189,6 @@ __host__ __device__ constexpr int vol_pad(int n) {
   return (NP == 8 && LPW == 0)   ? n + 2 * (n >> 4) + 2 * (n >> 6)
          : (NP == 4 && LPW == 0) ? n + 4 * (n >> 4)
          : (NP == 5 && LPW == 4) ? n + n / 5 + 5 * (n / 25)
-         : (NP == 6 && LPW == 4) ? n + 2 * (n / 36)
          : (NP == 7 && LPW == 4) ? n + n / 49
          : (NP == 3 && LPW == 8) ? n + 2 * (n >> 4)
                                  : vol_slot(n);
@@ -202,7 +201,7 @@ __host__ __device__ constexpr int vol_pad_slots() { return vol_pad<NP, LPW>(NP *
 
 template <int NP, int VF, int EPB = vol_epb<NP>(), int LPW = 0>
 __host__ __device__ constexpr size_t vol_smem_bytes() {
-  return sizeof(double) * (size_t)(2 * NP * NP + EPB * (VolRec<VF>::RS + 5) * vol_pad_slots<NP, LPW>());
+  return sizeof(double) * (size_t)(NP * NP + EPB * (VolRec<VF>::RS + 5) * vol_pad_slots<NP, LPW>());
 }
 
 // Node epilogue of the volume kernels: from the split-form volume integral ut of node t of element e
@@ -293,20 +292,16 @@ volume_kernel(KParams P) {
   constexpr int RS = VolRec<VF>::RS, NF = VolRec<VF>::NF;
   static_assert(LPW > 0 ? (32 / LPW >= NP) : (32 % NP == 0), "a line must fit its lanes of one warp");
   extern __shared__ double smem[];
-  double* sDvs = smem;         // Dvolsurf(i,l) at [i*NP+l]
-  double* sDhat = sDvs + NPT;  // D_hat(i,l)
+  double* sDvs = smem;  // Dvolsurf(i,l) at [i*NP+l]
   // node phases: thread -> (element slot eb, node t); with PACK the threads past EPB*NP3 idle
   const bool nodeThread = threadIdx.x < EPB * NP3;
   const int eb = nodeThread ? threadIdx.x / NP3 : 0, t = nodeThread ? threadIdx.x - eb * NP3 : 0;
   const int e = blockIdx.x * EPB + eb;
   const bool valid = nodeThread && e < P.nElems;
   constexpr int NS = vol_pad_slots<NP, LPW>();
-  double* rec = sDhat + NPT + (size_t)eb * (RS + 5) * NS;  // [slot][RS]
+  double* rec = sDvs + NPT + (size_t)eb * (RS + 5) * NS;  // [slot][RS]
   double* acc = rec + (size_t)RS * NS;                     // [slot][5]
-  for (int z = threadIdx.x; z < NPT; z += blockDim.x) {
-    sDvs[z] = P.basis->Dvs[z];
-    sDhat[z] = P.basis->Dhat[z];
-  }
+  for (int z = threadIdx.x; z < NPT; z += blockDim.x) sDvs[z] = P.basis->Dvs[z];
   __shared__ int sE2S[EPB][12];  // the element's ElemToSide (side, flip per local side)
   if (P.pfTiles > 0 && threadIdx.x == 0) {  // the tile one wave ahead: its inputs into L2
     const size_t en = ((size_t)blockIdx.x + P.pfTiles) * EPB;
@@ -361,7 +356,7 @@ volume_kernel(KParams P) {
       if (!lv) { p = 0; Ln = 0; }
     }
     const int la = Ln % NP, lb = Ln / NP;
-    double* prec = sDhat + NPT + (size_t)pe * (RS + 5) * NS;
+    double* prec = sDvs + NPT + (size_t)pe * (RS + 5) * NS;
     double* pacc = prec + (size_t)RS * NS;
 #pragma unroll 1
     for (int dir = 0; dir < 3; ++dir) {
