@@ -42,24 +42,28 @@ constexpr int vol_shape_count(int NP) {
 // results do not depend on what else the process ran, nor on a timing.  A batch keeps solves of different
 // shapes in different groups, so an instance runs the shape that it would run alone.
 //
-// One shape per N, but for N = 3.  us per step, best of repeated legs of the time loop, EC-KEP flux unless said:
+// us per step, best of repeated legs of the time loop, EC-KEP flux unless said:
 //   N = 1: {16} as fast or faster at every size (40^3 Euler 636, {32} 662);
 //   N = 2: {8,10} (27^3 Euler 605; {8,8} 717, {4,8} 730; at 4^3 84, 89, 83);
-//   N = 4: {2,6} (16^3 Navier-Stokes 1065; {2,4} 1083, {1,4} 1305; at 4^3 158, 163, 155);
-//   N = 5: two nodes per thread, {1,10,4} (14^3 Euler 579; {2,10,2} 581, one node 731; at 4^3 113, 113, 98);
 //   N = 6: {1,4} (13^3 Euler 779; {1,4,1} 1097, {1,4,0,1} 784; at 4^3 104, 102, 103);
-//   N = 7: two nodes per thread (12^3 Navier-Stokes 1371, one node 1482; at 4^3 217, 210).
-// The shape that is faster on a few elements is not used there where it is much slower on many: the tiny
-// solves of a batch share one launch.
+//   N = 4, 5, 7: up to one element per SM the latency of one block is the kernel's time, and one element per
+//   block and one node per thread make it the shortest: N = 4 {1,4} (4^3 Euler 90; {2,6} 94, {2,4} 98),
+//   N = 5 one node (4^3 Euler 98, two nodes 113), N = 7 one node (5^3 Euler 128, two nodes 132).  Above,
+//   throughput counts: N = 4 {2,6} (16^3 Navier-Stokes 1065; {2,4} 1083, {1,4} 1305), N = 5 two nodes,
+//   {1,10,4} (14^3 Euler 579; {2,10,2} 581, one node 731), N = 7 two nodes (12^3 Navier-Stokes 1371, one
+//   node 1482);
 //   N = 3: one node per thread, {2}, up to a few waves (8^3 Euler 88, two nodes 104); two nodes, {1,16,16},
 //   above 2^20 nodes (40^3 Euler 2617, one node 2695; Kennedy-Gruber 2491, 2750; Navier-Stokes 5743, 5773),
 //   and from 2^18 for Euler (20^3 407, 414).  Between, where launches start while the last wave of their
 //   predecessor drains (pdl_mode), one node is faster for Navier-Stokes (20^3 858, 870) and for the longer
 //   records of standard DG, dealiased metrics and Ducros (20^3 Euler 420, 479).
+// N = 2 and 6 keep the shape for large solves on small ones too: it costs them 2 to 4 %, and the small solves
+// of a batch share one launch, where it gains 20 to 40 %.
 constexpr int vol_shape_rule(int NP, int VF, bool visc, int nElems) {
   if (NP == 4)
     return nElems > (1 << 14) || (nElems >= (1 << 12) && !visc && VF != 0 && VF != 1 && VF != 3) ? 1 : 2;
-  return NP == 2 ? 1 : 0;
+  const bool few = nElems <= 148;  // SMs
+  return NP == 2 ? 1 : (few && (NP == 5 || NP == 6) ? 2 : (few && NP == 8 ? 1 : 0));
 }
 
 }  // namespace fluxo
