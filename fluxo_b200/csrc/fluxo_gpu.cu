@@ -294,8 +294,16 @@ void build_basis_tables(int N, BasisTables& B) {
 //   up to 2^20 their drain is worth filling: N = 3 Euler 20^3 492 / 473 / 461, N = 7 10^3 533 / 512 / 489;
 //   above, the early blocks only take cache and shared memory from the running kernel: N = 7 32^3 22.7 ms
 //   without, 23.2 ms with PDL_DRAIN.
+// A single right-hand side, which the host waits for, gains less from PDL_TAIL: it keeps PDL_DRAIN where the
+// blocks of two kernels fit side by side, up to 10^4 nodes (us per call, TAIL / DRAIN: N = 3 Euler 4^3 21.6 /
+// 21.3, N = 4 4^3 23.6 / 22.4; N = 3 Navier-Stokes 6^3, 13.8 k nodes, 35.2 / 38.7), and, for the two kernels of
+// Euler, from 10^5 (N = 5 8^3 34.3 / 32.9, N = 7 6^3 37.0 / 35.8; N = 3 10^3, 64 k nodes, 25.1 / 26.4).
 constexpr size_t kPdlDrainNodes = (size_t)1 << 18, kPdlNodes = (size_t)1 << 20;
 int pdl_mode(size_t nodes) { return nodes > kPdlNodes ? PDL_OFF : (nodes >= kPdlDrainNodes ? PDL_DRAIN : PDL_TAIL); }
+int pdl_mode_single(size_t nodes, bool visc) {
+  const int m = pdl_mode(nodes);
+  return m == PDL_TAIL && (nodes <= 10000 || (!visc && nodes >= 100000)) ? PDL_DRAIN : m;
+}
 
 KParams base_params(fluxo_handle* h) {
   KParams P{};
@@ -902,6 +910,7 @@ int fluxo_gpu_dg_time_derivative(fluxo_handle* h, double t) {
   P.stage = 0;
   P.t = t;
   P.grad = h->dGrad;  // keep the volume gradients of this RHS for fluxo_gpu_get_gradients
+  if (P.pdl != PDL_OFF) P.pdl = pdl_mode_single((size_t)h->nOwn * h->NP * h->NP * h->NP, h->visc);
   if ((r = rhs(h, P))) return r;
   FLUXO_CUDA(h, cudaStreamSynchronize(h->stream));
   FLUXO_CUDA(h, cudaGetLastError());
