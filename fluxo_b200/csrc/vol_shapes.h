@@ -45,25 +45,23 @@ constexpr int vol_shape_count(int NP) {
 // us per step, best of repeated legs of the time loop, EC-KEP flux unless said:
 //   N = 1: {16} as fast or faster at every size (40^3 Euler 636, {32} 662);
 //   N = 2: {8,10} (27^3 Euler 605; {8,8} 717, {4,8} 730; at 4^3 84, 89, 83);
+//   N = 4: {2,6} (16^3 Navier-Stokes 1065; {2,4} 1083, {1,4} 1305; at 4^3 158, 163, 155);
 //   N = 6: {1,4} (13^3 Euler 779; {1,4,1} 1097, {1,4,0,1} 784; at 4^3 104, 102, 103);
-//   N = 4, 5, 7: up to one element per SM the latency of one block is the kernel's time, and one element per
-//   block and one node per thread make it the shortest: N = 4 {1,4} (4^3 Euler 90; {2,6} 94, {2,4} 98),
-//   N = 5 one node (4^3 Euler 98, two nodes 113), N = 7 one node (5^3 Euler 128, two nodes 132).  Above,
-//   throughput counts: N = 4 {2,6} (16^3 Navier-Stokes 1065; {2,4} 1083, {1,4} 1305), N = 5 two nodes,
-//   {1,10,4} (14^3 Euler 579; {2,10,2} 581, one node 731), N = 7 two nodes (12^3 Navier-Stokes 1371, one
-//   node 1482);
+//   N = 7: two nodes per thread (12^3 Navier-Stokes 1371, one node 1482; at 4^3 217, 210);
+//   N = 5: two nodes per thread, {1,10,4} (14^3 Euler 579; {2,10,2} 581, one node 731), but one node, whose
+//   chain per thread is shorter, below 4^3 elements (3^3 Euler 96, two nodes 112; at 4^3 98, 113);
 //   N = 3: one node per thread, {2}, up to a few waves (8^3 Euler 88, two nodes 104); two nodes, {1,16,16},
 //   above 2^20 nodes (40^3 Euler 2617, one node 2695; Kennedy-Gruber 2491, 2750; Navier-Stokes 5743, 5773),
 //   and from 2^18 for Euler (20^3 407, 414).  Between, where launches start while the last wave of their
 //   predecessor drains (pdl_mode), one node is faster for Navier-Stokes (20^3 858, 870) and for the longer
 //   records of standard DG, dealiased metrics and Ducros (20^3 Euler 420, 479).
-// N = 2 and 6 keep the shape for large solves on small ones too: it costs them 2 to 4 %, and the small solves
-// of a batch share one launch, where it gains 20 to 40 %.
+// On a few dozen elements some shapes are 2 to 10 % faster than the one that is best on many.  They are not
+// used there: the small solves of a batch share a launch, and with shapes and groups of their own for up to
+// 148 elements at N = 4, 5 and 7 a batch of 64 solves (4^3 to 16^3 elements) took 20.2 instead of 18.7 ms a step.
 constexpr int vol_shape_rule(int NP, int VF, bool visc, int nElems) {
   if (NP == 4)
     return nElems > (1 << 14) || (nElems >= (1 << 12) && !visc && VF != 0 && VF != 1 && VF != 3) ? 1 : 2;
-  const bool few = nElems <= 148;  // SMs
-  return NP == 2 ? 1 : (few && (NP == 5 || NP == 6) ? 2 : (few && NP == 8 ? 1 : 0));
+  return NP == 2 ? 1 : (NP == 6 && nElems < 64 ? 2 : 0);
 }
 
 }  // namespace fluxo

@@ -38,8 +38,8 @@ def steps(N, eqn, elems):
 # N, eqn, elements of a small and a large solve, the shapes of both
 CASES = [(3, 0, (2, 2, 2), (16, 16, 16), 2, 1), (3, 0, (15, 16, 17), (16, 16, 16), 2, 1),
          (3, 1, (2, 2, 2), (16, 16, 16), 2, 2), (3, 1, (2, 2, 2), (26, 26, 25), 2, 1),
-         (5, 0, (2, 2, 2), (12, 12, 12), 2, 0), (5, 1, (4, 37, 1), (149, 1, 1), 2, 0),
-         (7, 1, (1, 1, 1), (8, 8, 8), 1, 0), (4, 1, (2, 2, 2), (10, 10, 10), 2, 0), (6, 0, (1, 1, 2), (6, 6, 6), 0, 0)]
+         (5, 0, (2, 2, 2), (12, 12, 12), 2, 0), (5, 1, (7, 9, 1), (4, 4, 4), 2, 0),
+         (7, 1, (1, 1, 1), (8, 8, 8), 0, 0), (4, 1, (2, 2, 2), (10, 10, 10), 0, 0), (6, 0, (1, 1, 2), (6, 6, 6), 0, 0)]
 
 
 @pytest.mark.parametrize("N,eqn,small,large,i_small,i_large", CASES)
