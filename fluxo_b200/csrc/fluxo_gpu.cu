@@ -288,17 +288,18 @@ void build_basis_tables(int N, BasisTables& B) {
 }
 
 // How early the launches of an Euler / Navier-Stokes solve of `nodes` own nodes start (PDL_*, common.cuh).
-// us per step without / PDL_TAIL / PDL_DRAIN, at the best launch shape of each:
-//   up to 2^18 nodes the kernels are a wave or two: N = 3 Euler 8^3 elements 117 / 88 / 107, N = 7
-//   Navier-Stokes 5^3 260 / 215 / 290 (N = 1 16^3: 193 / 146 / 224), N = 5 8^3 319 / 271 / 301;
-//   up to 2^20 their drain is worth filling: N = 3 Euler 20^3 492 / 473 / 461, N = 7 10^3 533 / 512 / 489;
+// us per step without / PDL_TAIL / PDL_DRAIN, at the launch shape that runs:
+//   below 200 k nodes the kernels are a wave or two: N = 3 Euler 8^3 elements 117 / 88 / 107, N = 7
+//   Navier-Stokes 5^3 260 / 221 / 290, N = 1 16^3 193 / 152 / 224, N = 5 8^3 321 / 278 / 307;
+//   up to 2^20 their drain is worth filling: N = 4 Navier-Stokes 12^3 519 / 486 / 483, N = 3 Euler 20^3
+//   494 / 477 / 461, N = 7 Euler 10^3 533 / 512 / 489;
 //   above, the early blocks only take cache and shared memory from the running kernel: N = 7 32^3 22.7 ms
 //   without, 23.2 ms with PDL_DRAIN.
 // A single right-hand side, which the host waits for, gains less from PDL_TAIL: it keeps PDL_DRAIN where the
 // blocks of two kernels fit side by side, up to 10^4 nodes (us per call, TAIL / DRAIN: N = 3 Euler 4^3 21.6 /
 // 21.3, N = 4 4^3 23.6 / 22.4; N = 3 Navier-Stokes 6^3, 13.8 k nodes, 35.2 / 38.7), and, for the two kernels of
 // Euler, from 10^5 (N = 5 8^3 34.3 / 32.9, N = 7 6^3 37.0 / 35.8; N = 3 10^3, 64 k nodes, 25.1 / 26.4).
-constexpr size_t kPdlDrainNodes = (size_t)1 << 18, kPdlNodes = (size_t)1 << 20;
+constexpr size_t kPdlDrainNodes = 200000, kPdlNodes = (size_t)1 << 20;
 int pdl_mode(size_t nodes) { return nodes > kPdlNodes ? PDL_OFF : (nodes >= kPdlDrainNodes ? PDL_DRAIN : PDL_TAIL); }
 int pdl_mode_single(size_t nodes, bool visc) {
   const int m = pdl_mode(nodes);
