@@ -57,11 +57,11 @@ LIFT_FLUX_BYTES_PER_POINT = 16 * 8
 # ncu figures of the shipped kernels.  DRAM bytes (read + write) per DOF of one launch of this
 # workload at its full size (32^3, one-pass capture of one time step's stages >= 2,
 # profiles/launches_dram_ns_tgv_N7_32x32x32.md); the FP64 pipe's active fraction
-# (sm__pipe_fp64_cycles_active, --set full on the 16^3 case, profiles/*_ns_tgv_N7_16x16x16.md), which
+# (sm__pipe_fp64_cycles_active on the 16^3 case, profiles/*_ns_tgv_N7_16x16x16.md), which
 # the F_alg fraction sits below where a kernel spends FP64 instructions that F_alg counts as one flop
 # (division, logarithm) or issues products and sums that a multiply-add would fuse.
-NCU_DRAM_BYTES_PER_DOF = {"volume": 321.0, "gradient": 209.1, "face_flux": 107.9, "lift_flux": 47.8}
-NCU_FP64_PIPE_ACTIVE = {"volume": 0.458, "gradient": 0.204, "face_flux": 0.372}  # gradient: DMMA tiles 0.119 more
+NCU_DRAM_BYTES_PER_DOF = {"volume": 310.8, "gradient": 209.4, "face_flux": 107.9, "lift_flux": 47.8}
+NCU_FP64_PIPE_ACTIVE = {"volume": 0.329, "gradient": 0.204, "face_flux": 0.372}  # gradient: DMMA tiles 0.119 more
 VOLUME_KERNEL_DRAM_BYTES_PER_DOF = NCU_DRAM_BYTES_PER_DOF["volume"]
 
 METRIC = "PID ns/DOF/RHS, NS Taylor-Green N=7 32^3 curved, BR1 + EC-KEP + ES (Riemann 44), LSERK4-5"
@@ -418,7 +418,7 @@ def run_fluxo(args):
     vol_avg_ms = vol_ms / max(vol_n, 1)
     vol_falg = MHD_VOLUME_KERNEL_FALG if mhd else VOLUME_KERNEL_FALG
     achieved = vol_falg * nd / (vol_avg_ms * 1e-3) / 1e12
-    roofline = {"bound": "fp64", "kernel": "mhd::volume_kernel<5,10>" if mhd else "volume_kernel<8,5,true>",
+    roofline = {"bound": "fp64", "kernel": "mhd::volume_kernel<5,10,1>" if mhd else volume_kernel_name(w["N"]),
                 "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                 "traffic": None if mhd else VOLUME_KERNEL_DRAM_BYTES_PER_DOF * nd,
                 "traffic_note": None if mhd else "DRAM bytes per launch, one-pass ncu capture of this workload",
@@ -492,7 +492,7 @@ def kernel_rooflines(kinds, N, nd, nElems, fp64_peak):
     bw, bw_src = hbm_peak()
     npts = 3 * nElems * (N + 1) ** 2
     out = {}
-    for k, name, falg in (("volume", "volume_kernel<%d,5,true>" % (N + 1), VOLUME_KERNEL_FALG),
+    for k, name, falg in (("volume", volume_kernel_name(N), VOLUME_KERNEL_FALG),
                           ("gradient", "lift_visc_mma_kernel<1,3>" if N == 7 else "lift_visc_kernel<%d,1,3>" % (N + 1),
                            LIFTING_KERNEL_FALG)):
         ms, n = kinds.get(k, (0.0, 0))
@@ -513,6 +513,12 @@ def kernel_rooflines(kinds, N, nd, nElems, fp64_peak):
     return out
 
 
+def volume_kernel_name(N):
+    """The Navier-Stokes volume kernel that ran: 64/(N+1) lines per warp mark the two-node one."""
+    blk = N in (3, 5, 7) and shape_dict(N, 5, True)["lines_per_warp"] == 64 // (N + 1)
+    return ("volume_blk_kernel<%d,5,1>" if blk else "volume_kernel<%d,5,1>") % (N + 1)
+
+
 def shape_dict(N, volume_flux, visc):
     """The volume kernel's launch shape of the last launch (index -1: none)."""
     from fluxo_b200.solver import volume_shape
@@ -527,11 +533,19 @@ def batch_falg(specs):
                for s in specs)
 
 
+def batch_groups(specs):
+    """The batch's groups: one per equation, N and launch shape of the volume kernel (vol_shape_rule of
+    csrc/vol_shapes.h for the mix's flux)."""
+    def few_or_many(eqn, N, n):
+        return n > 16384 or (n >= 4096 and eqn == 0) if N == 3 else N == 5 and n < 64
+
+    return {(s["eqn"], s["N"], few_or_many(s["eqn"], s["N"], s["elems"] ** 3)) for s in specs}
+
+
 def batch_launches_per_step(specs):
     """Kernels in one replay of the batch's step graph: per group reset, CALCTIMESTEP, dt, time update,
     and per stage face + volume (+ lifting flux + gradients for Navier-Stokes)."""
-    groups = {(s["eqn"], s["N"]) for s in specs}
-    return sum(4 + 5 * (4 if eqn == 1 else 2) for eqn, _ in groups)
+    return sum(4 + 5 * (4 if eqn == 1 else 2) for eqn, _, _ in batch_groups(specs))
 
 
 def run_batch(args):
@@ -557,7 +571,7 @@ def measure_batch(args, world, rank, local, steps=None):
     from fluxo_b200.workloads import batch_instance_specs, build_instance, instance_fields
 
     dev = torch.device("cuda", local)
-    nsteps = steps or nsteps
+    nsteps = steps or args.steps
     t0 = time.time()
     specs = batch_instance_specs(args.instances)
     cache, insts = {}, []
@@ -590,6 +604,7 @@ def measure_batch(args, world, rank, local, steps=None):
     ms_max = max_over_ranks(ms, world, dev)
     value = world * nd * 5 * nsteps / (ms_max * 1e-3)
     groups, placed, nbytes = b.info()
+    assert groups == len(batch_groups(specs)), groups
 
     # ---- end to end through the public API: host state in and out every step ----
     e2e = None

@@ -411,28 +411,29 @@ volume_kernel(KParams P) {
 
 // ------------------------------------------------------------------------------------------------
 // Volume kernel for even N+1 in {4, 6, 8}: the same sums as volume_kernel with two nodes of a line per
-// thread.  The one-node form waits on shared loads, shuffles and the chain of one pair flux at a time (FP64
-// pipe 46 % busy at N = 7): a pair takes ~20 shared loads and 10 32-bit shuffles there.  Here thread I of
-// the G = (N+1)/2 threads of a line holds nodes I and I+G in registers and meets the other threads' two
-// nodes at a time: its own pair first, then in round r = 1..(G-1)/2 the four pairs with the nodes of
-// thread I+r, and for even G a last round shared between the two threads of each opposite couple, two
-// pairs each.  A partner node's record is loaded once for two pairs and its sum shuffled back once, no
-// lane idles in a half-filled round, and the pairs are evaluated two at a time (pair_flux2).  One thread handles two nodes in the prologue
-// and epilogue as well; the metrics go to the records by asynchronous copies while the node's
-// quantities are formed (the pair fluxes that average two half metrics take whole ones and the
-// operator scaled by 1/2: exact).
+// thread.  The one-node form takes ~20 shared loads and 10 32-bit shuffles a pair and follows one pair flux at
+// a time.  Here thread I of the G = (N+1)/2 threads of a line holds nodes I and I+G in registers and meets
+// the other threads' two nodes at a time: its own pair first, then in round r = 1..(G-1)/2 the four pairs
+// with the nodes of thread I+r, and for even G a last round shared between the two threads of each opposite
+// couple, two pairs each.  A partner node's record is loaded once for two pairs and its sum shuffled back
+// once, no lane idles in a half-filled round, and the pairs are evaluated two at a time (pair_flux2): half the
+// shuffles for N+1 = 4 and 8, a third for 6; 272 shared loads a line for N+1 = 8 (EC-KEP) against 380, or 560
+// with the own record re-read in every round.  One thread handles two nodes in the prologue and epilogue as
+// well; the metrics go to the records by asynchronous copies while the node's quantities are formed (the
+// pair fluxes that average two half metrics take whole ones and the operator scaled by 1/2: exact).
 //
 // Measured, one B200, one-node form -> this one: Navier-Stokes N = 5 right-hand side (BR2, 463 k nodes) 228 ->
 // 204 us, N = 7 step (32^3 elements) 23.2 -> 22.7 ms, Euler N = 3 with subcells (512 k nodes, two steps) 1570 ->
-// 1486 us.  What bounds it now is latency again: 16 warps per SM at 128 registers, issue slots a third
-// busy, most stalls on the FP64 results of the own chain.  Where a mesh has too few elements to fill the
-// SMs (Euler N = 3, 512 elements) the one-node form's shorter chain per thread wins, so it stays among the
-// candidates of the launch-shape tuning (vol_shapes.h).
+// 1486 us.  What bounds it is the latency of global loads, then of the FP64 chains: 16 warps per SM at 128
+// registers, issue slots 38 % busy and the FP64 pipe 33 % at N = 7 (LSERK stage, 2.1 M nodes), per issue 3.7
+// warps waiting on global loads of the prologue and epilogue, 2.0 on a fixed latency, 0.6 on shared loads.
+// On few elements the one-node form's shorter chain per thread wins at N = 3 and 5 (vol_shape_rule, vol_shapes.h).
 //
 // Node slots (vb_slot) make every half-warp's 8-byte record and accumulator accesses hit 16 distinct
-// bank pairs, in the pair phase of all three directions and in the node phases: for N+1 = 8 and 4 a
-// permutation of the nodes whose low four bits differ over (position of thread I, lines of the
-// half-warp); the lines are dealt to warps in the order of vb_line.
+// bank pairs for N+1 = 8 and 4, in the pair phase of all three directions and in the node phases: a
+// permutation of the nodes whose low four bits differ over (position of thread I, lines of the half-warp);
+// the lines are dealt to warps in the order of vb_line.  N+1 = 6, one spare slot per plane, needs 1.6 times
+// the minimum in the pair phase.
 // ------------------------------------------------------------------------------------------------
 template <int NP>
 __host__ __device__ constexpr int vb_slot(int i, int j, int k) {

@@ -287,8 +287,8 @@ __host__ __device__ constexpr int epb() { return (256 / (NP * NP * NP)) > 0 ? (2
 
 // node slot of the records and accumulators: for N+1 = 5 (6 lines of 5 lanes per warp, 23-double
 // records) four spare slots after every 25 nodes, from a lane-by-lane model of the own, partner and
-// line-sum loads (1.12x the minimum shared wavefronts against 1.24x for one spare slot every 16
-// nodes); other N+1 keep the 16-node padding
+// accumulator accesses (1.58x the minimum of half-warp wavefronts against 1.79x for one spare slot
+// every 16 nodes); other N+1 keep the 16-node padding
 template <int NP>
 __host__ __device__ constexpr int mpad(int n) { return NP == 5 ? n + 4 * (n / 25) : vol_slot(n); }
 template <int NP>
